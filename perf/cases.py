@@ -1,0 +1,340 @@
+"""Performance cases of the framework on one GPU: what a user has it do, over the range of sizes it is used at.
+
+Kinds of work, each through the entry point that a program calls:
+
+* ``train``     ``Trainer.train_step`` with host batches in pinned memory: a whole optimizer step
+* ``score``     ``SimpleMoE.forward`` without gradients, tokens to logits (evaluation, scoring of ragged batches)
+* ``moe``       one ``MoEFFN`` block: router, dispatch, expert GEMMs, combine; forward, or forward and backward
+* ``experts``   ``ops.grouped_linear`` / ``ops.swiglu_probs`` on rows that are sorted by expert, in every precision recipe
+* ``head``      ``ops.linear_cross_entropy``: vocabulary projection and loss, with its gradients
+* ``exchange``  ``FusedDispatcher``: router selection, plan, dispatch of the token rows, gate-weighted combine
+
+Model shapes are those of ``system_lab_b200/models/presets.py``, cut to a few layers (and, where one GPU of an
+expert-parallel job would hold a part of the experts, to that part).  The widest one runs with grouped-query attention
+here: the library attention that latent attention falls back to cannot share a process with the others.
+"""
+from __future__ import annotations
+
+import math
+
+import torch
+
+from system_lab_b200 import ops
+from system_lab_b200.config import Config
+from system_lab_b200.moe.fused_dispatch import FusedDispatcher
+from system_lab_b200.parallel.mesh import single_process_mesh
+from system_lab_b200.pilot.constraints import param_counts
+from system_lab_b200.trainer.loop import Trainer, model_flops_per_token
+
+QWEN, OSS, DSV3, LLAMA = "qwen3-30b-a3b", "gpt-oss-20b", "deepseek-v3-proxy", "llama2-70b-lora"
+
+# hidden size, expert feed-forward size and experts on one GPU of the expert shapes
+EXPERT_SHAPES = {QWEN: (2048, 768, 128), OSS: (2880, 2880, 32), DSV3: (7168, 2048, 32)}
+TOPK = {QWEN: 8, OSS: 4, DSV3: 8}
+HEAD_SHAPES = {QWEN: (2048, 151936), OSS: (2880, 201088), DSV3: (7168, 129280), LLAMA: (8192, 32000)}
+
+
+def listed():
+    return [
+        # a debugging-size step (two narrow-vocabulary layers, 2 x 512 tokens): launches and host time dominate
+        dict(name="train-small", kind="train", preset=QWEN, layers=2, experts=16, vocab=4096, seq=512, mbs=2,
+             state="fp32", recompute="full", in_backward=False, fp8=""),
+        # the pretraining step as the headline benchmark runs it, at 4 of its 48 layers
+        dict(name="train-pretrain", kind="train", preset=QWEN, layers=4, experts=128, vocab=151936, seq=4096, mbs=2,
+             state="fp8", recompute="selective", in_backward=True, fp8=""),
+        # long sequences, head dim 64, a windowed and a full attention layer, hidden size that is no multiple of 128
+        dict(name="train-long-window", kind="train", preset=OSS, layers=2, experts=32, vocab=201088, seq=8192, mbs=1,
+             state="bf16", recompute="full", in_backward=True, fp8=""),
+        # the widest model: a dense and a MoE layer with a shared expert, block-scaled fp8 experts, sigmoid router
+        dict(name="train-wide-fp8", kind="train", preset=DSV3, layers=2, experts=32, vocab=129280, seq=4096, mbs=1,
+             state="fp8", recompute="selective", in_backward=True, fp8="blockwise"),
+        # low-rank fine-tuning of a dense layer on a batch of an odd length
+        dict(name="train-lora", kind="train", preset=LLAMA, layers=1, experts=0, vocab=32000, seq=2999, mbs=1,
+             state="fp32", recompute="selective", in_backward=False, fp8=""),
+        # evaluation: logits of three short sequences of an odd length
+        dict(name="score-ragged", kind="score", preset=QWEN, layers=2, experts=128, vocab=151936, seq=777, mbs=3),
+        # a handful of tokens through one MoE block: expert weights are read, little is multiplied
+        dict(name="moe-few-tokens", kind="moe", preset=QWEN, experts=128, tokens=61, backward=False),
+        # one MoE block of the wide model, 4096 tokens, forward and backward
+        dict(name="moe-wide", kind="moe", preset=DSV3, experts=32, tokens=4096, backward=True),
+        # expert GEMMs of a training step in the row-scaled fp8 recipe
+        dict(name="experts-fp8-rows", kind="experts", preset=DSV3, experts=32, slots=16384, zipf=False, fp8="rowwise",
+             backward=True),
+        # ... and forward only in the block-scaled recipe, skewed expert sizes
+        dict(name="experts-fp8-blocks", kind="experts", preset=DSV3, experts=32, slots=16384, zipf=True,
+             fp8="blockwise", backward=False),
+        # loss of a short ragged batch over a wide vocabulary, with gradients
+        dict(name="head-ragged", kind="head", preset=OSS, rows=1021, frozen=False),
+        # dispatch (fp8 payload) and combine of a full batch
+        dict(name="exchange", kind="exchange", hidden=7168, experts=256, topk=8, tokens=8192, zipf=False, fp8=True),
+    ]
+
+
+def _log_int(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def draw(rng):
+    kind = rng.choice(["train", "train", "score", "moe", "experts", "experts", "head", "exchange"])
+    if kind == "train":
+        preset = rng.choice([QWEN, OSS, DSV3, LLAMA])
+        c = dict(kind=kind, preset=preset, layers=rng.randint(1, 2), experts=0, vocab=rng.choice([4096, 32000, 64000]),
+                 seq=_log_int(rng, 100, 3000), mbs=rng.randint(1, 2), state=rng.choice(["fp32", "bf16", "fp8"]),
+                 recompute=rng.choice(["selective", "full"]), in_backward=rng.random() < 0.5, fp8="")
+        if preset != LLAMA:
+            c["experts"] = rng.choice([16, 32])
+            c["fp8"] = rng.choice(["", "rowwise", "blockwise", "tensorwise"])
+        else:
+            c["layers"], c["in_backward"] = 1, False
+        return c
+    if kind == "score":
+        return dict(kind=kind, preset=rng.choice([QWEN, OSS, DSV3]), layers=rng.randint(1, 2),
+                    experts=rng.choice([16, 32]), vocab=rng.choice([32000, 64000]), seq=_log_int(rng, 20, 2000),
+                    mbs=rng.randint(1, 3))
+    if kind == "moe":
+        preset = rng.choice([QWEN, OSS, DSV3])
+        return dict(kind=kind, preset=preset, experts=EXPERT_SHAPES[preset][2], tokens=_log_int(rng, 16, 4096),
+                    backward=rng.random() < 0.5)
+    if kind == "experts":
+        preset = rng.choice([QWEN, OSS, DSV3])
+        fp8 = "" if preset == OSS else rng.choice(["", "rowwise", "blockwise", "tensorwise"])
+        return dict(kind=kind, preset=preset, experts=rng.choice([8, EXPERT_SHAPES[preset][2]]),
+                    slots=_log_int(rng, 200, 20000), zipf=rng.random() < 0.5, fp8=fp8, backward=rng.random() < 0.5)
+    if kind == "head":
+        return dict(kind=kind, preset=rng.choice([QWEN, OSS, DSV3, LLAMA]), rows=_log_int(rng, 60, 4096),
+                    frozen=rng.random() < 0.3)
+    return dict(kind=kind, hidden=rng.choice([2048, 4096, 7168]), experts=rng.choice([32, 64, 128, 256]),
+                topk=rng.choice([2, 4, 8]), tokens=_log_int(rng, 50, 8192), zipf=rng.random() < 0.5,
+                fp8=rng.random() < 0.5)
+
+
+# ---------------------------------------------------------------------------------------------- set-up
+def _config(case, seed):
+    kind = case["kind"]
+    tokens = case.get("tokens")
+    ov = [f"num_layers={case.get('layers', 1)}", f"vocab_size={case.get('vocab', 1024)}",
+          f"seq_length={tokens or case['seq']}", f"micro_batch_size={case.get('mbs', 1)}",
+          f"global_batch_size={case.get('mbs', 1)}", "expert_model_parallel_size=1", "pipeline_model_parallel_size=1",
+          "device=cuda", f"seed={seed % (1 << 30)}", "clip_grad=1.0"]
+    if case["preset"] == DSV3:
+        ov += ["attention_type=gqa", "num_attention_heads=56", "num_query_groups=8", "kv_channels=128"]
+    if case["experts"]:
+        ov.append(f"num_experts={case['experts']}")
+    if kind == "train":
+        # a rate at which every step changes bf16 weights, and the first steps, without a warm-up, do not upset the model
+        ov += ["lr=1e-4", f"recompute_granularity={case['recompute']}", f"optimizer_state_dtype={case['state']}",
+               f"master_weights={'true' if case['state'] == 'fp32' else 'false'}",
+               f"optimizer_in_backward={'true' if case['in_backward'] else 'false'}",
+               f"fp8={'true' if case['fp8'] else 'false'}"]
+        if case["fp8"]:
+            ov.append(f"fp8_recipe={case['fp8']}")
+    elif kind == "score":
+        ov += ["recompute_granularity=selective", "fp8=false"]
+    else:
+        ov += ["recompute_granularity=none", "fp8=false", "first_k_dense=0", "moe_shared_expert_intermediate_size=0"]
+    return Config.load(preset=case["preset"], overrides=ov)
+
+
+def _trainer(case, seed):
+    return Trainer(_config(case, seed), mesh=single_process_mesh(), device=torch.device("cuda", torch.cuda.current_device()))
+
+
+def _tokens(vocab, mbs, seq, seed):
+    g = torch.Generator().manual_seed(seed)
+    t = torch.randint(0, vocab, (mbs, seq + 1), generator=g)
+    return t[:, :-1].contiguous(), t[:, 1:].contiguous()
+
+
+def _gpu_randn(shape, gen, std=1.0):
+    return torch.randn(shape, generator=gen, device="cuda", dtype=torch.bfloat16).mul_(std)
+
+
+def _segments(slots, experts, zipf, seed):
+    """Rows per expert of ``slots`` routed rows; every expert's rows start on a multiple of 128.  The seed says which
+    expert gets how many, out of one drawing of the counts (so that the padded total is the same for every seed)."""
+    p = 1.0 / torch.arange(1, experts + 1, dtype=torch.float64) ** (1.2 if zipf else 0.0)
+    hits = torch.multinomial(p / p.sum(), slots, replacement=True, generator=torch.Generator().manual_seed(slots))
+    counts = torch.bincount(hits, minlength=experts)[torch.randperm(experts, generator=torch.Generator().manual_seed(seed))]
+    padded = (counts + 127) // 128 * 128
+    return (torch.cumsum(padded, 0) - padded).int(), counts.int(), int(padded.sum())
+
+
+def prepare(case, seed):
+    kind = case["kind"]
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    s = {"case": case}
+    if kind == "train":
+        s["trainer"] = _trainer(case, seed)
+        tok, tgt = _tokens(case["vocab"], 8 * case["mbs"], case["seq"], seed)
+        tok, tgt = tok.pin_memory(), tgt.pin_memory()
+        s["batches"] = [[b] for b in zip(tok.split(case["mbs"]), tgt.split(case["mbs"]))]
+    elif kind == "score":
+        tr = s["trainer"] = _trainer(case, seed)
+        s["model"] = tr.engine.model.eval()
+        s["tokens"] = _tokens(case["vocab"], case["mbs"], case["seq"], seed)[0].cuda()
+    elif kind == "moe":
+        tr = s["trainer"] = _trainer(case, seed)
+        s["unit"], s["ffn"] = tr.engine.layer_units[0], tr.engine.moe_ffns()[0]
+        h = EXPERT_SHAPES[case["preset"]][0]
+        s["x"] = _gpu_randn((case["tokens"], h), gen).requires_grad_(case["backward"])
+        s["g"] = _gpu_randn((case["tokens"], h), gen)
+    elif kind == "experts":
+        h, f, _ = EXPERT_SHAPES[case["preset"]]
+        e = case["experts"]
+        off, cnt, rows = _segments(case["slots"], e, case["zipf"], seed)
+        # padding rows between the experts' segments are zero, as the dispatch leaves them
+        used = torch.zeros(rows, dtype=torch.bool)
+        for o, c in zip(off.tolist(), cnt.tolist()):
+            used[o:o + c] = True
+        used = used.cuda().unsqueeze(1)
+        s["offsets"], s["counts"] = off.cuda(), cnt.cuda()
+        grad = case["backward"]
+        s["x"] = _gpu_randn((rows, h), gen).mul_(used).requires_grad_(grad)
+        s["probs"] = torch.rand(rows, generator=gen, device="cuda").mul_(used.squeeze(1)).requires_grad_(grad)
+        s["g"] = _gpu_randn((rows, h), gen).mul_(used)
+        s["w1"] = _gpu_randn((e, 2 * f, h), gen, 0.02).requires_grad_(grad)
+        s["w2"] = _gpu_randn((e, h, f), gen, 0.02).requires_grad_(grad)
+    elif kind == "head":
+        h, v = HEAD_SHAPES[case["preset"]]
+        s["h"] = _gpu_randn((case["rows"], h), gen).requires_grad_(True)
+        s["w"] = _gpu_randn((v, h), gen, 0.02).requires_grad_(not case["frozen"])
+        s["targets"] = torch.randint(0, v, (case["rows"],), generator=gen, device="cuda")
+    else:
+        t, h, e, k = case["tokens"], case["hidden"], case["experts"], case["topk"]
+        s["d"] = FusedDispatcher(single_process_mesh(), e, k, h, t, 128, torch.device("cuda", torch.cuda.current_device()),
+                                 fp8_payload=case["fp8"])
+        s["x"] = _gpu_randn((t, h), gen)
+        s["logits"] = torch.randn(t, e, generator=gen, device="cuda")
+        if case["zipf"]:
+            s["logits"] -= 1.2 * torch.log(torch.arange(1, e + 1, device="cuda", dtype=torch.float32))
+        # what the expert GEMMs leave for the combine to collect
+        s["d"].expert_output_buffer().normal_(generator=gen)
+    return s
+
+
+# ---------------------------------------------------------------------------------------------- one pass
+def run(s):
+    return _RUN[s["case"]["kind"]](s)
+
+
+def _run_train(s):
+    tr = s["trainer"]
+    out = tr.train_step(batches=s["batches"][tr.step % len(s["batches"])])
+    return {"loss": out["loss"], "grad_norm": out["grad_norm"],
+            "weights": [g.shard for g in tr.engine.all_groups() if not g.frozen]}
+
+
+def _run_score(s):
+    with torch.no_grad():
+        return s["model"](s["tokens"], None, torch.bfloat16)
+
+
+def _run_moe(s):
+    if not s["case"]["backward"]:
+        with torch.no_grad():
+            return s["ffn"](s["x"])
+    s["unit"].prepare_grads()
+    s["x"].grad = None
+    y = s["ffn"](s["x"])
+    y.backward(s["g"])
+    ffn = s["ffn"]
+    return {"y": y.detach(), "dx": s["x"].grad, "dw1": ffn.experts_w1.main_grad, "dw2": ffn.experts_w2.main_grad,
+            "drouter": ffn.router.grad}
+
+
+def _run_experts(s):
+    case = s["case"]
+
+    def forward():
+        h1 = ops.grouped_linear(s["x"], s["w1"], s["offsets"], s["counts"], case["fp8"])
+        return ops.grouped_linear(ops.swiglu_probs(h1, s["probs"]), s["w2"], s["offsets"], s["counts"], case["fp8"])
+
+    if not case["backward"]:
+        with torch.no_grad():
+            return forward()
+    y = forward()
+    return (y.detach(),) + torch.autograd.grad(y, [s["x"], s["probs"], s["w1"], s["w2"]], s["g"])
+
+
+def _run_head(s):
+    loss = ops.linear_cross_entropy(s["h"], s["w"], s["targets"])
+    wanted = [s["h"]] + ([] if s["case"]["frozen"] else [s["w"]])
+    return (loss.detach(),) + torch.autograd.grad(loss, wanted)
+
+
+def _run_exchange(s):
+    d, case = s["d"], s["case"]
+    w, idx, _ = ops.router_fused(s["logits"], case["topk"])
+    plan = d.plan(idx)
+    if case["fp8"]:
+        d.scatter_ordered(plan, s["x"], w, 0, fp8=True).wait()
+        rows = [d.rows_fp8.view(torch.uint8), d.row_scales]
+    else:
+        rows = list(d.dispatch(plan, s["x"], w))
+    y = d.combine_rows(plan, d.expert_output_buffer(), w)
+    return [w, idx, y] + rows
+
+
+_RUN = {"train": _run_train, "score": _run_score, "moe": _run_moe, "experts": _run_experts, "head": _run_head,
+        "exchange": _run_exchange}
+
+
+# ---------------------------------------------------------------------------------------------- what a pass cannot do without
+_STATE_BYTES = {"fp32": 2 + 4 + 8, "bf16": 2 + 4, "fp8": 2 + 2 + 8 / 128}    # weights, master copy, two moments
+
+
+def work(case):
+    kind = case["kind"]
+    if kind in ("train", "score"):
+        m = _config(case, 0).model
+        pc = param_counts(m)
+        tokens = case["seq"] * case["mbs"]
+        if kind == "train":
+            flops = model_flops_per_token(m) * tokens
+            frozen = pc["total"] - pc["trainable"]
+            if frozen:
+                flops *= 2 / 3                                   # frozen matrices have no weight gradient
+            # every trainable parameter with its optimizer state is read and written, frozen ones are read
+            return {"bytes": 2 * _STATE_BYTES[case["state"]] * pc["trainable"] + 2 * frozen + 16 * tokens,
+                    "flops": flops}
+        return {"bytes": 2 * pc["total"] + 8 * tokens + 2 * tokens * case["vocab"],
+                "flops": model_flops_per_token(m) * tokens / 3}
+    if kind in ("moe", "experts"):
+        h, f, _ = EXPERT_SHAPES[case["preset"]]
+        e = case["experts"]
+        rows = case["tokens"] * TOPK[case["preset"]] if kind == "moe" else case["slots"]
+        io = case["tokens"] if kind == "moe" else rows           # rows read and written from outside
+        hit = e * (1 - (1 - 1 / e) ** rows)                      # experts that get a row at all
+        back = case["backward"]
+        # weights and input read and result written; backward: output gradient read, all gradients written
+        nbytes = hit * 6 * h * f + io * h * 2 * (4 if back else 2) + (e * 6 * h * f if back else 0)
+        return {"bytes": nbytes, "flops": (3 if back else 1) * 6 * rows * h * f}
+    if kind == "head":
+        h, v = HEAD_SHAPES[case["preset"]]
+        n, full = case["rows"], not case["frozen"]
+        return {"bytes": 2 * v * h * (2 if full else 1) + 4 * n * h + 8 * n, "flops": (6 if full else 4) * n * v * h}
+    t, h, k, e = case["tokens"], case["hidden"], case["topk"], case["experts"]
+    row = h + h // 32 if case["fp8"] else 2 * h
+    # tokens and logits read, one row per pair written; one row per pair read back, the result written
+    return {"bytes": 2 * t * h + 4 * t * e + t * k * row + 2 * t * k * h + 2 * t * h, "flops": 2 * t * k * h}
+
+
+def tolerance(case):
+    kind = case["kind"]
+    if kind == "train":
+        # Weights after a step.  The library attention's backward is not the same twice, and where a gradient is about
+        # zero Adam's step of one learning rate goes either way: after three steps two runs differ by 1.6e-3 in the norm
+        # of the weights, by 0.03 in a single weight and by 4e-4 in loss and gradient norm.
+        return {"rel": 6e-3, "max": 0.15}
+    if kind == "exchange":
+        # the payload's bytes are a rounding of the same rows; sums of top-k bf16 rows in fp32, stored in bf16
+        return {"rel": 4e-3, "max": 0.05, "differ": 1e-3}
+    if case.get("fp8"):
+        # e4m3 operands: against the fp32 oracle on the same quantised operands 2.5e-2 and 0.32, nearly all of it from
+        # activations that round to the neighbouring e4m3 value in the second GEMM's input
+        return {"rel": 0.03, "max": 0.9}
+    if kind == "score":
+        # bf16 through two layers; a token whose 8th and 9th expert score about the same may get the other one
+        return {"rel": 0.01, "max": 0.5}
+    # bf16 with fp32 sums, against the fp32 oracle: 1e-3 and 0.03 through both expert GEMMs
+    return {"rel": 4e-3, "max": 0.13}
