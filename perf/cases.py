@@ -319,6 +319,100 @@ def work(case):
     return {"bytes": 2 * t * h + 4 * t * e + t * k * row + 2 * t * k * h + 2 * t * h, "flops": 2 * t * k * h}
 
 
+def exact(case, seed):
+    """The same outputs in 64 bits.  Expert GEMMs in an fp8 recipe are compared with the product of their bf16 operands.
+    Whole models (``train``, ``score``) have none: rounding in one layer moves the routing of the next."""
+    kind = case["kind"]
+    if kind in ("train", "score"):
+        return None
+    s = prepare(case, seed)
+    if kind == "moe":
+        return _exact_moe(case, s)
+    if kind == "experts":
+        return _exact_experts(case, s)
+    if kind == "head":
+        return _exact_head(case, s)
+    w, idx = _exact_gates(s["logits"].double(), case["topk"], "softmax", True, 1.0)
+    flat = idx.reshape(-1)
+    counts = torch.bincount(flat, minlength=case["experts"])
+    padded = (counts + 127) // 128 * 128
+    start, first = torch.cumsum(padded, 0) - padded, torch.cumsum(counts, 0) - counts
+    order = torch.argsort(flat, stable=True)             # pairs by expert, in pair order inside an expert
+    rows = torch.empty_like(flat)
+    rows[order] = start[flat[order]] + torch.arange(flat.numel(), device="cuda") - first[flat[order]]
+    out = s["d"].expert_output_buffer()
+    y = torch.stack([(w[t] * out[r].double().movedim(-1, 0)).sum(-1)
+                     for t, r in enumerate(rows.view(idx.shape))])
+    return [w, None, y]
+
+
+def _exact_gates(logits, topk, score, norm, scaling):
+    """Gate weights (differentiable in the logits) and the experts that every token selects."""
+    scores = torch.softmax(logits, -1) if score == "softmax" else torch.sigmoid(logits)
+    w, idx = scores.topk(topk, -1)
+    return (w / w.sum(-1, keepdim=True) if norm else w) * scaling, idx
+
+
+def _exact_expert(x, probs, w1, w2, g):
+    """One expert on its rows: ``(y, dx, dprobs, dw1, dw2)``; gradients only with ``g``."""
+    x, probs, w1, w2 = (t.detach().double().requires_grad_(g is not None) for t in (x, probs, w1, w2))
+    gate, up = (x @ w1.t()).chunk(2, -1)
+    y = (torch.nn.functional.silu(gate) * up * probs.unsqueeze(-1)) @ w2.t()
+    if g is None:
+        return y, None, None, None, None
+    return (y.detach(),) + torch.autograd.grad(y, [x, probs, w1, w2], g.double())
+
+
+def _exact_experts(case, s):
+    back = case["backward"]
+    y = torch.zeros(s["x"].shape, dtype=torch.float64, device="cuda")
+    dx, dp = torch.zeros_like(y), torch.zeros(y.shape[0], dtype=torch.float64, device="cuda")
+    dw1, dw2 = (torch.zeros(s[w].shape, dtype=torch.float64, device="cuda") if back else None for w in ("w1", "w2"))
+    for e, (o, c) in enumerate(zip(s["offsets"].tolist(), s["counts"].tolist())):
+        r = slice(o, o + c)
+        got = _exact_expert(s["x"][r], s["probs"][r], s["w1"][e], s["w2"][e], s["g"][r] if back else None)
+        y[r] = got[0]
+        if back:
+            dx[r], dp[r], dw1[e], dw2[e] = got[1:]
+    return (y, dx, dp, dw1, dw2) if back else y
+
+
+def _exact_moe(case, s):
+    ffn, back = s["ffn"], case["backward"]
+    cfg = ffn.cfg
+    x = s["x"].detach().double().requires_grad_(True)
+    router = ffn.router.detach().double().requires_grad_(True)
+    w, idx = _exact_gates(x @ router.t(), cfg.moe_router_topk, cfg.moe_router_score_function, cfg.moe_norm_topk_prob,
+                          cfg.moe_router_topk_scaling_factor)
+    y, dx, dw = torch.zeros_like(x), torch.zeros_like(x), torch.zeros_like(w)
+    dw1 = torch.zeros(ffn.experts_w1.shape, dtype=torch.float64, device="cuda") if back else None
+    dw2 = torch.zeros(ffn.experts_w2.shape, dtype=torch.float64, device="cuda") if back else None
+    for e in range(cfg.num_experts):
+        t, k = torch.nonzero(idx == e, as_tuple=True)
+        got = _exact_expert(x[t], w[t, k], ffn.experts_w1[e], ffn.experts_w2[e], s["g"][t] if back else None)
+        with torch.no_grad():
+            y[t] += got[0]
+            if back:
+                dx[t] += got[1]
+                dw[t, k], dw1[e], dw2[e] = got[2:]
+    if not back:
+        return y.detach()
+    through_gates = torch.autograd.grad(w, [x, router], dw)
+    return {"y": y.detach(), "dx": dx.detach() + through_gates[0], "dw1": dw1, "dw2": dw2, "drouter": through_gates[1]}
+
+
+def _exact_head(case, s):
+    h, w, targets = s["h"].detach().double(), s["w"].detach().double(), s["targets"]
+    p = h @ w.t()
+    n = torch.arange(p.shape[0], device="cuda")
+    lse = torch.logsumexp(p, -1, keepdim=True)
+    loss = (lse.squeeze(-1) - p[n, targets]).mean()
+    p.sub_(lse).exp_()
+    p[n, targets] -= 1
+    p /= p.shape[0]
+    return (loss, p @ w) + (() if case["frozen"] else (p.t() @ h,))
+
+
 def tolerance(case):
     kind = case["kind"]
     if kind == "train":
