@@ -40,6 +40,17 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp, and a value all its lanes share.  TMA and tcgen05 instructions take their operands from uniform
+// registers.  In a branch on the thread index the compiler cannot know that one thread is there, and moves every operand
+// over at each instruction: about 130 cycles per issued copy or MMA.  Warps that issue them therefore run their loops
+// as a whole, on values that are visibly the same in all lanes, and elect the issuing lane at the instruction.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 // ---------------------------------------------------------------- mbarrier
@@ -71,7 +82,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // other waiter leaves on its next poll.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  // the clock is looked at only once a wait has turned out not to be one of the many short ones
+#pragma unroll 1
+  for (int i = 0; i < 32; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {

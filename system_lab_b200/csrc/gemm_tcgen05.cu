@@ -1,20 +1,19 @@
-// Dropless grouped expert GEMM for sm_100a: tcgen05.mma with TMEM accumulators, operands staged by
-// TMA (no cluster multicast), persistent warp-specialised CTAs.
+// Grouped expert GEMM fused with a transfer, one CTA per tile: tcgen05.mma with TMEM accumulators, operands staged by
+// TMA (no cluster multicast), persistent warp-specialised CTAs.  The plain products run on pairs of SMs (gemm_pair.cu);
+// this kernel is for results that are pushed to the rows' owners (PUSH) and for weights that are gathered while they are
+// multiplied (GATHER).
 //
 // Roles per CTA (192 threads): warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane, also
 // owns the TMEM allocation), warps 2..5 = epilogue (each drains its 32 TMEM lanes to global memory).
 // Two TMEM accumulators (2 x BN fp32 columns) let the epilogue of tile i overlap the main loop of
 // tile i+1.  All waits are bounded (see common.cuh).
 //
-// Three modes share one kernel; rows are grouped by expert, every segment starts at a multiple of 128
+// Two modes share one kernel; rows are grouped by expert, every segment starts at a multiple of 128
 // rows and padding rows are zero (the dispatch kernels guarantee both):
 //   FWD    C[r, n]   = sum_k A[r, k]  * B[e, n, k]      A: acts  [R, K]   B: weights [E, N, K]
 //   DGRAD  C[r, k]   = sum_n A[r, n]  * B[e, n, k]      A: dY    [R, N]   B: weights [E, N, K] (MN-major operand)
-//   WGRAD  C[e, n, k]= sum_r A[r, n]  * B[r, k]         A: dY    [R, N]   B: acts    [R, K]   (both MN-major,
-//                                                       reduction length = rows of expert e)
 // Reference analogue: the hand written MFMA grouped GEMM (128x128x32 tiles, double buffered LDS,
-// notes/2026-04/2026-04-10-mfma-gemm-optimization.md:35-109) and the variable-K wgrad kernel of
-// notes/2026-04/2026-04-21_gptoss_10_moe_fp8_grouped_gemm_diagnosis.md:64-85.
+// notes/2026-04/2026-04-10-mfma-gemm-optimization.md:35-109).
 #include "common.cuh"
 #include "tma_host.cuh"
 
@@ -25,7 +24,7 @@ constexpr int BK = 64;            // 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int GEMM_THREADS = 192;
 
-enum { MODE_FWD = 0, MODE_DGRAD = 1, MODE_WGRAD = 2 };
+enum { MODE_FWD = 0, MODE_DGRAD = 1 };
 
 struct GemmParams {
   const int* seg_offsets;   // [E] first row of each expert segment (multiple of 128)
@@ -35,7 +34,6 @@ struct GemmParams {
   int N;                    // weights' N
   int K;                    // weights' K
   __nv_bfloat16* C;
-  int accumulate;           // WGRAD: add into C instead of overwriting
   int* status;
   // push epilogue (FWD / DGRAD): every output row goes straight to the rank its token came from
   const int* origin;        // [R] (source rank << 24) | pair index, written by the senders' scatter
@@ -45,11 +43,7 @@ struct GemmParams {
   int world, me, epoch;
   int pairs;                // rows of the pair-major region (a row origin outside it is reported, not written)
   int* counter;             // CTAs that finished pushing (reset by the last one)
-  // per-(source, expert) arrival flags of the row operand A (FWD / DGRAD): the rows of expert e were written by
-  // `ready_world` sources, source s releases ready[s * E + e] = ready_epoch when its rows of e are complete
-  const int* ready;
-  int ready_world, ready_epoch;
-  unsigned long long ready_limit_ns;
+  unsigned long long wait_limit_ns;   // GATHER: bound of the waits on flags and piece counts
   // fused all-gather of the weight operand's flat buffer (GATHER, forward only): a seventh warp in every CTA pulls
   // this CTA's share of every piece of [0, g_bytes) of the flat parameter buffer from the ranks' staged shards
   // (plain 16-byte peer loads) and counts the piece; the TMA producer loads a weight tile only after the pieces
@@ -108,19 +102,11 @@ __device__ __forceinline__ bool get_tile(int t, const int* prefix, const GemmPar
   int e = lo;
   int local = t - prefix[e];
   ti.e = e;
-  if (MODE == MODE_WGRAD) {
-    int m_tiles = (p.N + BM - 1) / BM;        // output rows = weights' N (a partial last tile when N % 128 == 64)
-    ti.m_idx = local % m_tiles;
-    ti.n_idx = local / m_tiles;
-    ti.row0 = p.seg_offsets[e];
-    ti.ksteps = (seg_rows(p, e) + BK - 1) / BK;
-  } else {
-    int m_tiles = (seg_rows(p, e) + BM - 1) / BM;
-    ti.m_idx = local % m_tiles;
-    ti.n_idx = local / m_tiles;
-    ti.row0 = p.seg_offsets[e] + ti.m_idx * BM;
-    ti.ksteps = ((MODE == MODE_FWD) ? p.K : p.N) / BK;
-  }
+  int m_tiles = (seg_rows(p, e) + BM - 1) / BM;
+  ti.m_idx = local % m_tiles;
+  ti.n_idx = local / m_tiles;
+  ti.row0 = p.seg_offsets[e] + ti.m_idx * BM;
+  ti.ksteps = ((MODE == MODE_FWD) ? p.K : p.N) / BK;
   return true;
 }
 
@@ -135,7 +121,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
   using L = SmemLayout<BN>;
   constexpr int STAGES = L::STAGES;
-  constexpr bool A_MN = (MODE == MODE_WGRAD);
   constexpr bool B_MN = (MODE != MODE_FWD);
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {                 // swizzled tiles need a 1024-byte aligned base
@@ -173,7 +158,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     int acc = 0;
     for (int e = 0; e < p.E; ++e) {
       prefix[e] = acc;
-      int per = (MODE == MODE_WGRAD) ? ((p.N + BM - 1) / BM) : ((seg_rows(p, e) + BM - 1) / BM);
+      int per = (seg_rows(p, e) + BM - 1) / BM;
       acc += per * n_tiles;
     }
     prefix[p.E] = acc;
@@ -192,28 +177,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    // Lane 0 issues the copies.  When the row operand arrives from other GPUs expert by expert (`ready`), the whole
-    // warp first polls the flags of the tile's expert, one source per lane: the GEMM starts on an expert as soon as
-    // every source has delivered it, while rows of later experts are still in flight.  The rows were written by
-    // peers' generic-proxy stores; the proxy fence orders the TMA (async proxy) reads after the acquire.
+    // Lane 0 issues the copies; the whole warp waits for gathered weights.
     int s = 0;
     uint32_t ph = 0;
-    int last_e = -1;
     TileInfo ti;
     bool ok = true;
     for (int t = blockIdx.x; ok && get_tile<MODE, BN>(t, prefix, p, n_tiles, ti); t += gridDim.x) {
-      if (MODE != MODE_WGRAD && p.ready != nullptr && ti.e != last_e) {
-        bool mine = true;
-        if (lane < p.ready_world)
-          mine = wait_flag_ge(p.ready + lane * p.E + ti.e, p.ready_epoch, p.status, p.ready_limit_ns);
-        ok = __all_sync(0xffffffffu, mine);
-        if (!ok) {
-          if (lane == 0) *abort_flag = 1;
-          break;
-        }
-        asm volatile("fence.proxy.async.global;" ::: "memory");
-        last_e = ti.e;
-      }
       if (GATHER && MODE == MODE_FWD) {
         // the weight tile's bytes inside the flat buffer -> the pieces that cover them, one piece per lane
         const long t0 = p.g_w_off + ((long)ti.e * p.N + (long)ti.n_idx * BN) * p.K * 2;
@@ -223,7 +192,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int p0 = (int)(t0 / p.g_piece_bytes), p1 = (int)((t1 - 1) / p.g_piece_bytes);
         bool mine = true;
         for (int q = p0 + lane; q <= p1 && mine; q += 32) {
-          if (q < p.g_pieces) mine = wait_count_ge(p.g_piece_count + q, p.g_target, p.status, p.ready_limit_ns);
+          if (q < p.g_pieces) mine = wait_count_ge(p.g_piece_count + q, p.g_target, p.status, p.wait_limit_ns);
         }
         ok = __all_sync(0xffffffffu, mine);
         if (!ok) {
@@ -241,18 +210,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (MODE == MODE_FWD) {
             tma_load_2d(a_dst, &tmap_a, &full_bar[s], ks * BK, ti.row0);
             tma_load_2d(b_dst, &tmap_b, &full_bar[s], ks * BK, ti.e * p.N + ti.n_idx * BN);
-          } else if (MODE == MODE_DGRAD) {
+          } else {
             tma_load_2d(a_dst, &tmap_a, &full_bar[s], ks * BK, ti.row0);
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(b_dst + j * 8192, &tmap_b, &full_bar[s], ti.n_idx * BN + j * 64, ti.e * p.N + ks * BK);
-          } else {
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(a_dst + j * 8192, &tmap_a, &full_bar[s], ti.m_idx * BM + j * 64, ti.row0 + ks * BK);
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(b_dst + j * 8192, &tmap_b, &full_bar[s], ti.n_idx * BN + j * 64, ti.row0 + ks * BK);
           }
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -262,14 +224,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0, BM, BN);
+      constexpr uint32_t idesc = make_idesc(1, 1, 0, B_MN ? 1 : 0, BM, BN);
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
       TileInfo ti;
       bool ok = true;
       for (int t = blockIdx.x; ok && get_tile<MODE, BN>(t, prefix, p, n_tiles, ti); t += gridDim.x) {
-        if (ti.ksteps == 0) continue;
         const int buf = it & 1;
         if (!mbar_wait(&tempty_bar[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
@@ -282,8 +243,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
           for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
             // K-major: 32 bytes per UMMA_K inside the 128-byte swizzle row; MN-major: 16 k-rows of 128 bytes
-            const uint64_t adesc = A_MN ? make_smem_desc(a_addr + k4 * 2048, 8192, 1024, 2)
-                                        : make_smem_desc(a_addr + k4 * 32, 16, 1024, 2);
+            const uint64_t adesc = make_smem_desc(a_addr + k4 * 32, 16, 1024, 2);
             const uint64_t bdesc = B_MN ? make_smem_desc(b_addr + k4 * 2048, 8192, 1024, 2)
                                         : make_smem_desc(b_addr + k4 * 32, 16, 1024, 2);
             umma_f16(d_tmem, adesc, bdesc, idesc, (ks | k4) != 0 ? 1u : 0u);
@@ -299,7 +259,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else if (GATHER && warp == 6) {
     // ------------------------------------------------------------ gather warp (see GemmParams)
     bool good = true;
-    if (lane < p.g_world) good = wait_flag_ge(p.g_ready + lane, p.g_epoch, p.status, p.ready_limit_ns);
+    if (lane < p.g_world) good = wait_flag_ge(p.g_ready + lane, p.g_epoch, p.status, p.wait_limit_ns);
     good = __all_sync(0xffffffffu, good);
     // One warp per CTA moves this CTA's share of a piece in units of 512 bytes (32 lanes x 16 bytes), GU units at a
     // time: all GU peer loads of a lane are issued before the first store, so a lane keeps GU x 16 bytes in flight
@@ -347,8 +307,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     // TMEM -> registers -> bf16 -> swizzled shared staging (64 columns at a time, two buffers) -> TMA store.
-    // Rows/columns outside the output tensor are clipped by the TMA unit.  The accumulate variant of wgrad
-    // (beta = 1) reads and writes global memory directly instead.
+    // Rows/columns outside the output tensor are clipped by the TMA unit.
     const int lg = warp & 3;                    // TMEM lane group this warp may read
     const bool store_thread = (warp == 2 && lane == 0);
     const int r_in_tile = lg * 32 + lane;
@@ -358,15 +317,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     TileInfo ti;
     for (int t = blockIdx.x; get_tile<MODE, BN>(t, prefix, p, n_tiles, ti); t += gridDim.x) {
       const int col0 = ti.n_idx * BN;
-      const int tile_row = (MODE == MODE_WGRAD) ? (ti.e * p.N + ti.m_idx * BM) : ti.row0;
-      // wgrad tiles that accumulate (beta = 1), or that hang over the end of an expert's N rows (the 2-D output map
-      // cannot clip at an expert boundary), go through guarded global loads / stores instead of the TMA store
-      const bool partial = (MODE == MODE_WGRAD) && (ti.m_idx * BM + BM > p.N);
-      const bool direct = (MODE == MODE_WGRAD) && (p.accumulate || partial);
-      __nv_bfloat16* c_row = p.C + (size_t)(tile_row + r_in_tile) * out_cols;
-      const bool row_ok = (MODE == MODE_WGRAD) ? (ti.m_idx * BM + r_in_tile < p.N) : (tile_row + r_in_tile < p.R);
-      const bool empty = (ti.ksteps == 0);      // expert without rows (wgrad): the gradient is zero
-      if (empty && direct && p.accumulate) continue;
+      const int tile_row = ti.row0;
+      const bool row_ok = tile_row + r_in_tile < p.R;
       int* org_tile = origin_s + (tile_ctr & 1) * BM;
       if (PUSH) {
         // padding rows of the segment have no owner; the table is double buffered because a warp may start the
@@ -375,48 +327,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         org_tile[r_in_tile] = (r_in_tile < valid && row_ok) ? p.origin[tile_row + r_in_tile] : -1;
         ++tile_ctr;
       }
-      int buf = 0;
-      if (!empty) {
-        buf = it & 1;
-        if (!mbar_wait(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) break;
-        tc_fence_after();
-      }
+      const int buf = it & 1;
+      if (!mbar_wait(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) break;
+      tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * BN;
 #pragma unroll 1
       for (int c = 0; c < BN; c += 64) {
         uint32_t v[64];
-        if (!empty) {
-          uint32_t lo[32], hi[32];
-          tmem_ld_32x32(taddr + c, lo);
-          tmem_ld_32x32(taddr + c + 32, hi);
-          tmem_ld_wait();
+        uint32_t lo[32], hi[32];
+        tmem_ld_32x32(taddr + c, lo);
+        tmem_ld_32x32(taddr + c + 32, hi);
+        tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) { v[i] = lo[i]; v[32 + i] = hi[i]; }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = 0u;
-        }
-        if (direct) {
-          if (row_ok) {
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const int col = col0 + c + g * 8;
-              if (col < out_cols) {
-                float f[8], o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]);
-                bf16x8* dst = reinterpret_cast<bf16x8*>(c_row + col);
-                if (p.accumulate) {
-                  unpack8(*dst, o);
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) f[i] += o[i];
-                }
-                *dst = pack8(f);
-              }
-            }
-          }
-          continue;
-        }
+        for (int i = 0; i < 32; ++i) { v[i] = lo[i]; v[32 + i] = hi[i]; }
         uint8_t* sb = store_buf + (chunk_ctr & 1) * L::STORE_BYTES;
         // the TMA store that last read this buffer (two chunks ago) must have finished reading it
         if (!PUSH && store_thread) tma_store_wait_read<1>();
@@ -457,12 +380,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         ++chunk_ctr;
       }
-      if (!empty) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[buf]);
-        ++it;
-      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+      ++it;
     }
     if (PUSH) {
       // completion: every thread fences its peer stores, the last CTA releases this rank's flag on every peer
@@ -506,18 +427,13 @@ static int launch(const void* A, const void* B, const GemmParams& p, int grid, c
   if (MODE == MODE_FWD) {
     if ((rc = tma_make_map_bf16(&ma, A, p.R, p.K, BM, BK))) return rc;
     if ((rc = tma_make_map_bf16(&mb, B, (uint64_t)p.E * p.N, p.K, BN, BK))) return rc;
-  } else if (MODE == MODE_DGRAD) {
+  } else {
     if ((rc = tma_make_map_bf16(&ma, A, p.R, p.N, BM, BK))) return rc;
     if ((rc = tma_make_map_bf16(&mb, B, (uint64_t)p.E * p.N, p.K, BK, 64))) return rc;
-  } else {
-    if ((rc = tma_make_map_bf16(&ma, A, p.R, p.N, BK, 64))) return rc;
-    if ((rc = tma_make_map_bf16(&mb, B, p.R, p.K, BK, 64))) return rc;
   }
   CUtensorMap mc;
   if (PUSH) {
     mc = ma;                                  // the push epilogue stores with plain peer writes: no output map
-  } else if (MODE == MODE_WGRAD) {
-    if ((rc = tma_make_map_bf16(&mc, p.C, (uint64_t)p.E * p.N, p.K, BM, 64))) return rc;
   } else {
     if ((rc = tma_make_map_bf16(&mc, p.C, p.R, (MODE == MODE_FWD) ? p.N : p.K, BM, 64))) return rc;
   }
@@ -533,40 +449,7 @@ static int launch(const void* A, const void* B, const GemmParams& p, int grid, c
 
 }  // namespace slab
 
-// mode: 0 fwd, 1 dgrad, 2 wgrad.  Shapes: see the header comment.  Requires K % 64 == 0, N % 64 == 0
-// (wgrad: a last partial row tile is written with guarded stores), at most 512 experts.  `status` is a device int
-// the kernel sets on a
-// bounded-wait timeout (0 = ok).  Returns a CUDA/driver error code (0 = launched).
-// `ready` (optional, modes 0 and 1): per-(source, expert) arrival flags of the row operand, int [ready_world][E] in
-// this GPU's memory; the kernel waits (bounded) for all `ready_world` flags of an expert to reach `ready_epoch`
-// before it loads that expert's first row tile.  Null: the operand is complete when the kernel starts.
 extern "C" unsigned long long slab_moe_wait_limit_ns();
-
-extern "C" int slab_grouped_gemm_bf16(int mode, const void* A, const void* B, void* C, const int* seg_offsets,
-                                      const int* seg_counts, int E, int R, int N, int K, int accumulate,
-                                      int block_n, int max_ctas, const int* ready, int ready_world, int ready_epoch,
-                                      int* status, cudaStream_t stream) {
-  using namespace slab;
-  if (E > 512 || K % 64 || N % 64) return -100;
-  if (ready && (ready_world < 1 || ready_world > 32 || mode == MODE_WGRAD)) return -102;
-  GemmParams p{seg_offsets, seg_counts, E, R, N, K, static_cast<__nv_bfloat16*>(C), accumulate, status};
-  p.ready = ready;
-  p.ready_world = ready_world;
-  p.ready_epoch = ready_epoch;
-  p.ready_limit_ns = slab_moe_wait_limit_ns();
-  int grid = sm_count();
-  if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
-  const bool wide = block_n != 128;
-  switch (mode) {
-    case MODE_FWD:
-      return wide ? launch<MODE_FWD, 256>(A, B, p, grid, stream) : launch<MODE_FWD, 128>(A, B, p, grid, stream);
-    case MODE_DGRAD:
-      return wide ? launch<MODE_DGRAD, 256>(A, B, p, grid, stream) : launch<MODE_DGRAD, 128>(A, B, p, grid, stream);
-    case MODE_WGRAD:
-      return wide ? launch<MODE_WGRAD, 256>(A, B, p, grid, stream) : launch<MODE_WGRAD, 128>(A, B, p, grid, stream);
-  }
-  return -101;
-}
 
 // Forward (mode 0) or dgrad (mode 1) whose result rows are pushed to the ranks that own the rows' tokens instead
 // of being stored locally.  `origin[r]` = (source rank << 24) | pair index for every valid row, `peer_ptrs` the
@@ -581,8 +464,7 @@ extern "C" int slab_grouped_gemm_bf16_push(int mode, const void* A, const void* 
   using namespace slab;
   if (E > 256 || K % 64 || N % 64 || world > 16 || world < 1 || me < 0 || me >= world) return -100;
   if (mode != MODE_FWD && mode != MODE_DGRAD) return -101;
-  GemmParams p{seg_offsets, seg_counts, E, R, N, K, nullptr, 0, status};
-  p.ready = nullptr;
+  GemmParams p{seg_offsets, seg_counts, E, R, N, K, nullptr, status};
   p.origin = origin;
   for (int i = 0; i < 16; ++i) p.peer[i] = i < world ? reinterpret_cast<uint8_t*>(peer_ptrs[i]) : nullptr;
   p.comb_off = comb_off;
@@ -628,7 +510,7 @@ extern "C" int slab_dense_gemm_gather(const void* A, void* C, const int* seg_off
   p.K = K;
   p.C = static_cast<__nv_bfloat16*>(C);
   p.status = status;
-  p.ready_limit_ns = slab_moe_wait_limit_ns();
+  p.wait_limit_ns = slab_moe_wait_limit_ns();
   const long ready_off = layout[0], ack_off = layout[1], slots_off = layout[2], slot_bytes = layout[3];
   for (int r = 0; r < 16; ++r) {
     p.g_src[r] = r < world ? reinterpret_cast<const uint8_t*>(peer_ptrs[r]) + slots_off + (long)slot * slot_bytes : nullptr;

@@ -23,7 +23,7 @@ from collections import defaultdict
 
 # (category, substrings) — first match wins; names are lower-cased first.
 RULES: list[tuple[str, tuple[str, ...]]] = [
-    ("slab_grouped_gemm", ("grouped_gemm_kernel", "grouped_gemm_fp8")),
+    ("slab_grouped_gemm", ("grouped_gemm_kernel", "grouped_gemm_fp8", "pair_gemm_kernel")),
     ("slab_dispatch", ("moe_scatter_kernel", "moe_combine", "moe_count", "moe_publish", "moe_plan", "moe_slots",
                        "moe_wait", "moe_signal", "moe_reduce", "moe_check", "moe_gather")),
     ("slab_norm", ("rmsnorm_fwd_kernel", "rmsnorm_bwd_kernel", "colsum_to_bf16")),

@@ -1,0 +1,89 @@
+"""Grouped GEMM on pairs of SMs at the sizes where its tiles end: chunks of rows, output blocks, reduction remainders."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(counts, n, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    cnt = torch.tensor(counts, dtype=torch.int32)
+    pad = (cnt + 127) // 128 * 128
+    off, rows = torch.cumsum(pad, 0) - pad, max(int(pad.sum()), 128)
+    used = torch.zeros(rows, 1, device="cuda")
+    for o, c in zip(off.tolist(), counts):
+        used[o:o + c] = 1
+    a = (torch.randn(rows, k, generator=g, device="cuda") * used).bfloat16()
+    dy = (torch.randn(rows, n, generator=g, device="cuda") * used).bfloat16()
+    w = (0.05 * torch.randn(len(counts), n, k, generator=g, device="cuda")).bfloat16()
+    return a, dy, w, off.int().cuda(), cnt.cuda()
+
+
+def _close(out, ref, magnitude):
+    """bf16 result of an fp32 sum: half a bf16 step of the value (2^-9), doubled for sums that round across a binade, and
+    2^-20 of the summed magnitudes for the order of the sum."""
+    from system_lab_b200.ops import cuda
+    cuda.check_status()
+    bound = ref.abs() * 2 ** -8 + magnitude * 2 ** -20 + 1e-30
+    assert bool(((out.double() - ref).abs() <= bound).all()), float(((out.double() - ref).abs() / bound).max())
+
+
+# rows around the 32-row unit, the 256-row chunk and uneven cuts; output columns around the 64-, 128- and 256-wide blocks
+SIZES = [([1], 64, 64), ([31, 32, 33], 64, 192), ([255, 256, 257], 192, 128), ([0, 513, 0, 5], 320, 64),
+         ([1100, 3], 128, 320), ([700] * 9, 576, 448), ([2] * 400, 64, 128)]
+
+
+@pytest.mark.parametrize("counts,n,k", SIZES)
+def test_rows_against_64_bits(counts, n, k):
+    from system_lab_b200.ops import cuda
+    a, dy, w, off, cnt = _operands(counts, n, k, 1)
+    for mode, x, cols in ((0, a, n), (1, dy, k)):
+        out = torch.full((x.shape[0], cols), float("nan"), device="cuda", dtype=torch.bfloat16)
+        cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k, out=out)
+        for e, (o, c) in enumerate(zip(off.tolist(), counts)):
+            we = w[e].double().t() if mode == 0 else w[e].double()
+            _close(out[o:o + c], x[o:o + c].double() @ we, x[o:o + c].double().abs() @ we.abs())
+            assert not bool(out[o + c:o + (c + 127) // 128 * 128].any())     # padding rows are zero
+
+
+@pytest.mark.parametrize("counts,n,k", SIZES)
+def test_weight_gradient_against_64_bits(counts, n, k):
+    from system_lab_b200.ops import cuda
+    a, dy, w, off, cnt = _operands(counts, n, k, 2)
+    out = torch.full_like(w, float("nan"))
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=out)
+    twice = w.clone()
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=twice, accumulate=True)
+    for e, (o, c) in enumerate(zip(off.tolist(), counts)):
+        d, x = dy[o:o + c].double(), a[o:o + c].double()
+        _close(out[e], d.t() @ x, d.abs().t() @ x.abs())
+        _close(twice[e], w[e].double() + d.t() @ x, w[e].double().abs() + d.abs().t() @ x.abs())
+
+
+@pytest.mark.parametrize("rows", [1, 33, 100, 1021])
+def test_one_segment_that_ends_inside_a_tile(rows):
+    from system_lab_b200.ops import cuda
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(rows, 192, generator=g, device="cuda").bfloat16()
+    w = torch.randn(1, 320, 192, generator=g, device="cuda").bfloat16()
+    off, cnt = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((1,), rows, dtype=torch.int32, device="cuda")
+    guard = torch.full((rows + 64, 320), 7.0, device="cuda", dtype=torch.bfloat16)
+    cuda.grouped_gemm_raw(0, x, w, off, cnt, 320, 192, out=guard[:rows])
+    _close(guard[:rows], x.double() @ w[0].double().t(), x.double().abs() @ w[0].double().abs().t())
+    assert bool((guard[rows:] == 7).all())
+    dw = cuda.grouped_gemm_raw(2, guard[:rows], x, off, cnt, 320, 192)[0]
+    _close(dw, guard[:rows].double().t() @ x.double(), guard[:rows].double().abs().t() @ x.double().abs())
+
+
+@pytest.mark.parametrize("counts,n,k", [([1], 64, 128), ([31, 0, 257], 192, 256), ([700, 130], 320, 768)])
+def test_row_scaled_e4m3(counts, n, k):
+    from system_lab_b200.ops import cuda
+    a, _, w, off, cnt = _operands(counts, n, k, 4)
+    aq, sa = cuda.quant_rowwise(a)
+    wq, sw = cuda.quant_rowwise(w)
+    out = cuda.grouped_gemm_fp8_rowwise_raw(aq, sa, wq, sw.contiguous(), off, cnt)
+    for e, (o, c) in enumerate(zip(off.tolist(), counts)):
+        x = aq[o:o + c].double() * sa[o:o + c, None].double()
+        m = (wq[e].double() * sw[e][:, None].double()).t()
+        # the tensor core adds e4m3 products with fewer bits than fp32 (2^-13 of the summed magnitudes at most)
+        _close(out[o:o + c], x @ m, (x.abs() @ m.abs()) * 2 ** 7)
