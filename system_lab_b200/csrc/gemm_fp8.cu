@@ -9,6 +9,10 @@
 // columns).  Operands arrive by TMA (128-byte swizzle: one 128-element fp8 row per swizzle row), 6 stages,
 // no cluster multicast.  The output goes through swizzled shared staging and a TMA store.
 //
+// Bound by the read-out and scaling of a partial tile per K block (two columns per multiply-add).  Copies and MMAs are
+// issued by an elected lane of a converged warp; before, issuing them was what a K block waited for: 32 experts, 16384 rows,
+// 7168 -> 4096 782 -> 588 us (1230 -> 1637 TFLOP/s), 2048 -> 7168 408 -> 313 us, the same bits.
+//
 // Reference analogues: the fused fp8 grouped GEMM with dequantising epilogue (`acc *= sa*sb`,
 // summary/fp8_expert_gemm_optimization.md:84-116) and the blockwise recipe that was the slowest variant there
 // (notes/2026-04/2026-04-21_gptoss_10_moe_fp8_grouped_gemm_diagnosis.md:74-85).
@@ -25,6 +29,20 @@ constexpr int F8_STORE_OFF = F8_CTRL + F8_STAGES * F8_STAGE;
 constexpr int F8_STORE_BYTES = F8_BM * 64 * 2;
 constexpr int F8_SMEM = F8_STORE_OFF + 2 * F8_STORE_BYTES;
 static_assert(F8_SMEM <= 232448, "shared memory budget");
+
+constexpr int F8_AHEAD = 4;              // K blocks whose scales are requested ahead
+
+// two fp32 values side by side: one instruction multiplies and adds both
+__device__ __forceinline__ unsigned long long f32x2(uint32_t lo, uint32_t hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
 
 struct Fp8Params {
   const int* seg_offsets;
@@ -78,7 +96,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   int* prefix = reinterpret_cast<int*>(smem + F8_PREFIX_OFF);
   uint8_t* ring = smem + F8_CTRL;
   uint8_t* store_buf = smem + F8_STORE_OFF;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n_tiles = (p.N + F8_BN - 1) / F8_BN;
   const int kblocks = p.K / F8_BK;
 
@@ -104,51 +122,56 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int tiles = warp_uniform(prefix[p.E]);
 
   if (warp == 0) {
-    if (lane == 0) {                                   // ---------------- TMA producer
-      int s = 0;
-      uint32_t ph = 0;
+    // ---------------- TMA producer (the whole warp, see elect_one)
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
       F8Tile ti;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && f8_get_tile(t, prefix, p, ti); t += gridDim.x) {
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-          uint8_t* a_dst = ring + s * F8_STAGE;
+      f8_get_tile(t, prefix, p, ti);
+      const int a_row = warp_uniform(ti.row0), b_row = warp_uniform(ti.e * p.N + ti.n_idx * F8_BN);
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY));
+        if (!ok) break;
+        uint8_t* a_dst = ring + s * F8_STAGE;
+        if (elect_one()) {
           mbar_arrive_expect_tx(&full_bar[s], F8_STAGE);
-          tma_load_2d(a_dst, &tmap_a, &full_bar[s], kb * F8_BK, ti.row0);
-          tma_load_2d(a_dst + F8_A_BYTES, &tmap_b, &full_bar[s], kb * F8_BK, ti.e * p.N + ti.n_idx * F8_BN);
-          if (++s == F8_STAGES) { s = 0; ph ^= 1; }
+          tma_load_2d(a_dst, &tmap_a, &full_bar[s], kb * F8_BK, a_row);
+          tma_load_2d(a_dst + F8_A_BYTES, &tmap_b, &full_bar[s], kb * F8_BK, b_row);
         }
+        if (++s == F8_STAGES) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {                                   // ---------------- MMA issuer: one TMEM buffer per K block
-      constexpr uint32_t idesc = make_idesc(0, 0, 0, 0, F8_BM, F8_BN);     // e4m3 x e4m3, K-major both
-      int s = 0;
-      uint32_t ph = 0;
-      uint32_t it = 0;                                 // K blocks issued so far (selects the TMEM buffer)
-      F8Tile ti;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && f8_get_tile(t, prefix, p, ti); t += gridDim.x) {
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const uint32_t buf = it % F8_TBUF;
-          if (!mbar_wait(&tempty_bar[buf], ((it / F8_TBUF) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(ring + s * F8_STAGE);
-          const uint32_t b_addr = a_addr + F8_A_BYTES;
+    // ---------------- MMA issuer: one TMEM buffer per K block
+    constexpr uint32_t idesc = make_idesc(0, 0, 0, 0, F8_BM, F8_BN);     // e4m3 x e4m3, K-major both
+    const uint64_t a0 = make_smem_desc(smem_u32(ring), 16, 1024, 2);
+    const uint64_t b0 = make_smem_desc(smem_u32(ring) + F8_A_BYTES, 16, 1024, 2);
+    int s = 0;
+    uint32_t ph = 0;
+    uint32_t it = 0;                                   // K blocks issued so far (selects the TMEM buffer)
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+      for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        const uint32_t buf = it % F8_TBUF;
+        ok = __all_sync(0xffffffffu,
+                        mbar_wait(&tempty_bar[buf], ((it / F8_TBUF) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY) &&
+                            mbar_wait(&full_bar[s], ph, abort_flag, p.status, ST_TIMEOUT_FULL));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-          for (int k4 = 0; k4 < F8_BK / F8_UK; ++k4) {
-            const uint64_t adesc = make_smem_desc(a_addr + k4 * 32, 16, 1024, 2);
-            const uint64_t bdesc = make_smem_desc(b_addr + k4 * 32, 16, 1024, 2);
-            umma_f8(tmem_base + buf * F8_BN, adesc, bdesc, idesc, k4 != 0 ? 1u : 0u);
-          }
+          for (int k4 = 0; k4 < F8_BK / F8_UK; ++k4)
+            umma_f8(tmem_base + buf * F8_BN, a0 + (uint32_t)(s * (F8_STAGE >> 4)) + k4 * 2,
+                    b0 + (uint32_t)(s * (F8_STAGE >> 4)) + k4 * 2, idesc, k4 != 0 ? 1u : 0u);
           umma_commit(&empty_bar[s]);
           umma_commit(&tfull_bar[buf]);
-          if (++s == F8_STAGES) { s = 0; ph ^= 1; }
         }
+        if (++s == F8_STAGES) { s = 0; ph ^= 1; }
       }
     }
   } else {
@@ -164,15 +187,26 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     F8Tile ti;
     bool ok = true;
     for (int t = blockIdx.x; ok && f8_get_tile(t, prefix, p, ti); t += gridDim.x) {
-      float acc[64];
+      unsigned long long acc[32];                        // two fp32 columns each
 #pragma unroll
-      for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+      for (int i = 0; i < 32; ++i) acc[i] = 0ull;
       const int row = ti.row0 + r_in_tile;
       const float* sa_row = p.sa + (size_t)(row < p.R ? row : 0) * kblocks;
       const float* sb_row = p.sb + ((size_t)ti.e * nb_total + ti.n_idx) * kblocks;
+      auto scale_at = [&](int kb) {
+        return kb < kblocks ? (row < p.R ? __ldg(sa_row + kb) : 0.f) * __ldg(sb_row + kb) : 0.f;
+      };
+      // The lanes' activation scales lie a row apart, 32 cache lines per load, and the operand ring leaves the L1 too small
+      // to keep them: every load goes to L2.  They are requested F8_AHEAD K blocks ahead.
+      float sc[F8_AHEAD];
+#pragma unroll
+      for (int i = 0; i < F8_AHEAD; ++i) sc[i] = scale_at(i);
       for (int kb = 0; kb < kblocks; ++kb, ++it) {
         const uint32_t buf = it % F8_TBUF;
-        const float sc = (row < p.R ? __ldg(sa_row + kb) : 0.f) * __ldg(sb_row + kb);
+        const float now = sc[0];
+#pragma unroll
+        for (int i = 0; i + 1 < F8_AHEAD; ++i) sc[i] = sc[i + 1];
+        sc[F8_AHEAD - 1] = scale_at(kb + F8_AHEAD);
         if (!mbar_wait(&tfull_bar[buf], (it / F8_TBUF) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * F8_BN + half * 64;
@@ -183,10 +217,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);     // the MMA warp may refill this buffer during the FMAs
+        const unsigned long long s2 = f32x2(__float_as_uint(now), __float_as_uint(now));
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          acc[i] = fmaf(__uint_as_float(v0[i]), sc, acc[i]);
-          acc[32 + i] = fmaf(__uint_as_float(v1[i]), sc, acc[32 + i]);
+        for (int i = 0; i < 16; ++i) {
+          acc[i] = fma_f32x2(f32x2(v0[2 * i], v0[2 * i + 1]), s2, acc[i]);
+          acc[16 + i] = fma_f32x2(f32x2(v1[2 * i], v1[2 * i + 1]), s2, acc[16 + i]);
         }
       }
       if (!ok) break;
@@ -197,7 +232,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       for (int g = 0; g < 8; ++g) {
         float f[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = acc[g * 8 + i];
+        for (int i = 0; i < 4; ++i) {
+          f[2 * i] = __uint_as_float((uint32_t)acc[g * 4 + i]);
+          f[2 * i + 1] = __uint_as_float((uint32_t)(acc[g * 4 + i] >> 32));
+        }
         *reinterpret_cast<bf16x8*>(sbuf + r_in_tile * 128 + ((g ^ (r_in_tile & 7)) << 4)) = pack8(f);
       }
       fence_proxy_async();
