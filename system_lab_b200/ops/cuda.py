@@ -34,6 +34,7 @@ _SIGS = {
     "slab_router_fused_fwd": "ppppiiiiifpfps",
     "slab_router_fused_bwd": "pppppfpiiiiifs",
     "slab_ce_fwd_bwd": "pppiifs",
+    "slab_quant_tensorwise": "ppppls",
     "slab_grouped_gemm_bf16": "i" + "p" * 5 + "i" * 7 + "pii" + "ps",
     "slab_grouped_gemm_fp8": "p" * 7 + "iiiii" + "ps",
     "slab_grouped_gemm_fp8_rowwise": "p" * 7 + "iiiii" + "ps",
@@ -80,7 +81,7 @@ def _ptr(t):
 
 
 # kernels launched per entry point (entry points not listed launch one); LAUNCHES[0] counts launches
-_KERNELS_PER_CALL = {}
+_KERNELS_PER_CALL = {"slab_quant_tensorwise": 2}
 LAUNCHES = [0]
 
 
@@ -456,7 +457,8 @@ def grouped_gemm_raw(mode: int, a, b, offsets, counts, n: int, k: int, out=None,
 
     ``ready`` (modes 0 and 1): arrival flags of the row operand (an object with ``flags`` int32 [world, E], ``world``,
     ``epoch`` and ``mark_consumed()``): the kernel waits per expert for every source instead of the caller waiting
-    for the whole exchange."""
+    for the whole exchange.  ``block_n`` is the tile width of the one-CTA kernel behind pushed results; the kernel here
+    picks its own tiles."""
     e = offsets.numel()
     r = a.shape[0]
     if out is None:
@@ -857,11 +859,16 @@ def linear_cross_entropy(h, weight, targets, chunk_rows: int = 8192):
 
 
 # ------------------------------------------------------------------------------ quantisation
+def _aligned16(x):
+    """``x`` where a kernel may read it 16 bytes at a time (a view can start anywhere in its storage)."""
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 def quant_1x128(x):
     if not _bf16(x):
         return ref.quant_1x128(x)
     shp = x.shape
-    x2 = x.reshape(-1, shp[-1]).contiguous()
+    x2 = _aligned16(x.reshape(-1, shp[-1]).contiguous())
     q = torch.empty(x2.shape, dtype=torch.float8_e4m3fn, device=x.device)
     s = torch.empty(x2.shape[0], shp[-1] // 128, dtype=torch.float32, device=x.device)
     call("slab_quant_1x128", x2, q, s, x2.shape[0], shp[-1], stream())
@@ -882,8 +889,14 @@ def quant_rowwise(x):
 
 def quant_tensorwise(x):
     """e4m3 with a single fp32 scale for the whole tensor (current scaling: the scale comes from this tensor's own
-    absolute maximum, no history).  Library elementwise kernels; the row-scaled recipe is the fused one."""
-    return ref.quant_tensorwise(x)
+    absolute maximum, no history): returns ``(q, scale 0-d)``."""
+    if not _bf16(x) or not x.is_cuda or x.numel() == 0:
+        return ref.quant_tensorwise(x)
+    xc = _aligned16(x.detach().contiguous())
+    q = torch.empty(xc.shape, dtype=torch.float8_e4m3fn, device=x.device)
+    s = torch.empty((), dtype=torch.float32, device=x.device)
+    call("slab_quant_tensorwise", xc, q, s, torch.zeros(1, dtype=torch.int32, device=x.device), xc.numel(), stream())
+    return q, s
 
 
 def quant_128x128(w):
