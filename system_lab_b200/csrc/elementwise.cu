@@ -605,6 +605,25 @@ quant_tensorwise_kernel(const bf16x8* __restrict__ x, uint2* __restrict__ q, lon
         __nv_fp8_e4m3(__fdiv_rn(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[rest]), sc));
 }
 
+// x *= g, nothing to do where g is one (the usual gradient of a loss): 1.16 GB of vocabulary gradient cost 657 us as a library
+// product, 2 us now.  16 bytes per thread, x 16-byte aligned.
+__global__ void __launch_bounds__(256)
+scale_bf16_kernel(bf16x8* __restrict__ x, long n, const float* __restrict__ g) {
+  const float s = __bfloat162float(__float2bfloat16_rn(*g));
+  if (s == 1.f) return;
+  const long nvec = n >> 3;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nvec; i += (long)gridDim.x * blockDim.x) {
+    float f[8];
+    unpack8(x[i], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] *= s;
+    x[i] = pack8(f);
+  }
+  const long rest = (nvec << 3) + threadIdx.x;
+  __nv_bfloat16* xe = reinterpret_cast<__nv_bfloat16*>(x);
+  if (blockIdx.x == 0 && rest < n) xe[rest] = __float2bfloat16_rn(__bfloat162float(xe[rest]) * s);
+}
+
 // ------------------------------------------------------------------ squared L2 norm (fp32 input)
 template <typename G>
 __global__ void sumsq_kernel(const G* __restrict__ g, long n, float scale, float* __restrict__ out) {
@@ -964,6 +983,13 @@ extern "C" int slab_quant_tensorwise(const void* x, void* q, float* scale, unsig
   const int grid = grid_for((nvec + 3) / 4, 256);
   amax_bf16_kernel<<<grid, 256, 0, st>>>((const uint4*)x, nvec, (const unsigned short*)x + nvec * 8, (int)(n - nvec * 8), mag);
   quant_tensorwise_kernel<<<grid, 256, 0, st>>>((const bf16x8*)x, (uint2*)q, n, mag, scale);
+  return (int)cudaGetLastError();
+}
+
+// x (bf16, 16-byte aligned) times the fp32 scalar *g rounded to bf16, in place.
+extern "C" int slab_scale_bf16(void* x, long n, const float* g, cudaStream_t st) {
+  if (n == 0) return 0;
+  scale_bf16_kernel<<<grid_for(n / 8 + 1, 256), 256, 0, st>>>((bf16x8*)x, n, g);
   return (int)cudaGetLastError();
 }
 

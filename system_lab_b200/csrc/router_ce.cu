@@ -284,70 +284,119 @@ router_fused_bwd_kernel(const float* __restrict__ logits, const int* __restrict_
   }
 }
 
-// One block per row: loss_row = logsumexp(logits) - logits[target]; logits <- (softmax - onehot) * gscale.
-// `loss_sum` accumulates sum of row losses (fp32 atomics).  V % 8 == 0.
-__global__ void __launch_bounds__(512)
-ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, float* __restrict__ loss_sum,
-                  int rows, int V, float gscale) {
-  __shared__ float red[32];
-  __shared__ float bc[2];
+// CTAS blocks (a cluster) per row: loss_row = logsumexp(logits) - logits[target]; logits <- (softmax - onehot) * gscale
+// (GRAD).  `loss_sum` accumulates sum of row losses (fp32 atomics).  V % 8 == 0.
+//
+// Bound by memory and the exponentials (two per element on a pipe of 16 lanes per clock).  A row is 2 V bytes (300 - 400 KB
+// at the vocabularies in use), too long for one SM's shared memory, so it is read twice.  The maximum and the sum come
+// from ONE pass (running maximum, rescaled sum), and few rows are in flight at a time, so the second read and the write
+// find the row in the 126 MB L2 and memory sees one read and one write.  Long rows are shared by the two blocks of a
+// cluster: 148 rows of at most 400 KB = 60 MB in flight, and every SM has blocks of two rows, one of which computes while
+// the other waits at a row's end.  The next piece is requested before the current one is worked on.  [1021, 201088] 297 ->
+// 227 us (3.6 TB/s of one read and one write), the loss alone 105; [8192, 151936] 1553 -> 1292 us, 573; three reads before.
+constexpr int CE_UNROLL = 2;
+
+template <int CTAS>
+__device__ __forceinline__ void ce_row_sync() {
+  if (CTAS > 1)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  else
+    __syncthreads();
+}
+// the other block's copy of a shared variable
+__device__ __forceinline__ float ce_peer(const float* v, uint32_t peer) {
+  uint32_t a;
+  float f;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(v)), "r"(peer));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(a) : "memory");
+  return f;
+}
+
+// Calls f(vector, index) for the vectors lo + threadIdx.x, + THREADS, ... below hi.
+template <int THREADS, typename F>
+__device__ __forceinline__ void ce_walk(const bf16x8* row, int lo, int hi, F f) {
+  bf16x8 next[CE_UNROLL];
+#pragma unroll
+  for (int u = 0; u < CE_UNROLL; ++u)
+    if (lo + (int)threadIdx.x + u * THREADS < hi) next[u] = row[lo + threadIdx.x + u * THREADS];
+  for (int c0 = lo + threadIdx.x; c0 < hi; c0 += THREADS * CE_UNROLL) {
+    bf16x8 v[CE_UNROLL];
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u) {
+      v[u] = next[u];
+      const int c = c0 + (CE_UNROLL + u) * THREADS;
+      if (c < hi) next[u] = row[c];
+    }
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u)
+      if (c0 + u * THREADS < hi) f(v[u], c0 + u * THREADS);
+  }
+}
+
+template <int THREADS, int CTAS, bool GRAD>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
+ce_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, float* __restrict__ loss_sum, int rows,
+          int V, float gscale) {
+  __shared__ float red_m[2][THREADS / 32], red_s[2][THREADS / 32];   // by parity of the row: one barrier per row
+  __shared__ float all_m[2], all_s[2];
+  constexpr int WARPS = THREADS / 32;
   const int nvec = V >> 3;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = CTAS > 1 ? (int)(blockIdx.x % CTAS) : 0;
+  const int half = (nvec + CTAS - 1) / CTAS;
+  const int lo = rank * half, hi = min(nvec, lo + half);
+  int par = 0;
+  for (int r = blockIdx.x / CTAS; r < rows; r += gridDim.x / CTAS, par ^= 1) {
     bf16x8* row = reinterpret_cast<bf16x8*>(logits + (size_t)r * V);
-    float mx = -INFINITY;
-    for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
-      float f[8];
-      unpack8(row[c], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) mx = fmaxf(mx, f[j]);
-    }
-    mx = warp_max(mx);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : -INFINITY;
-      t = warp_max(t);
-      if (threadIdx.x == 0) bc[0] = t;
-    }
-    __syncthreads();
-    mx = bc[0];
-    float sum = 0.f;
-    for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
-      float f[8];
-      unpack8(row[c], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sum += __expf(f[j] - mx);
-    }
-    sum = warp_sum(sum);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-      t = warp_sum(t);
-      if (threadIdx.x == 0) bc[1] = t;
-    }
-    __syncthreads();
-    sum = bc[1];
     const long tgt = targets[r];
-    if (threadIdx.x == 0) {
-      float lt = __bfloat162float(logits[(size_t)r * V + tgt]);
-      atomicAdd(loss_sum, logf(sum) + mx - lt);
-    }
-    __syncthreads();        // the target logit is read before anyone overwrites it
-    const float inv = gscale / sum;
-    for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+    const float lt = threadIdx.x == 0 ? __bfloat162float(logits[(size_t)r * V + tgt]) : 0.f;
+    float m = -INFINITY, s = 0.f;
+    ce_walk<THREADS>(row, lo, hi, [&](const bf16x8& v, int) {
       float f[8];
-      unpack8(row[c], f);
+      unpack8(v, f);
+      float vm = f[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) vm = fmaxf(vm, f[j]);
+      if (vm > m) {
+        s *= __expf(m - vm);               // the first time m is -inf and s is 0
+        m = vm;
+      }
+      // columns masked with -inf: while nothing finite was seen the reference point is 0, and they add exp(-inf) = 0
+      const float ref = m == -INFINITY ? 0.f : m;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += __expf(f[j] - ref);
+    });
+    const float wm = warp_max(m);
+    s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));
+    if (lane == 0) { red_m[par][warp] = wm; red_s[par][warp] = s; }
+    __syncthreads();
+    const float bm = lane < WARPS ? red_m[par][lane] : -INFINITY;
+    const float bs = lane < WARPS ? red_s[par][lane] : 0.f;
+    float mx = warp_max(bm);
+    float sum = warp_sum(bm == -INFINITY ? bs : bs * __expf(bm - mx));
+    if (CTAS > 1) {
+      if (threadIdx.x == 0) { all_m[par] = mx; all_s[par] = sum; }
+      ce_row_sync<CTAS>();                 // both parts have been read and summed
+      const float pm = ce_peer(&all_m[par], rank ^ 1), ps = ce_peer(&all_s[par], rank ^ 1);
+      const float top = fmaxf(mx, pm);
+      sum = (mx == -INFINITY ? sum : sum * __expf(mx - top)) + (pm == -INFINITY ? ps : ps * __expf(pm - top));
+      mx = top;
+    }
+    if (rank == 0 && threadIdx.x == 0) atomicAdd(loss_sum, logf(sum) + mx - lt);
+    if (!GRAD) continue;
+    const float inv = gscale / sum;
+    ce_walk<THREADS>(row, lo, hi, [&](const bf16x8& v, int c) {
+      float f[8];
+      unpack8(v, f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         f[j] = __expf(f[j] - mx) * inv;
         if ((long)c * 8 + j == tgt) f[j] -= gscale;
       }
       row[c] = pack8(f);
-    }
+    });
   }
+  if (CTAS > 1) ce_row_sync<CTAS>();       // the other block may still be reading this one's sums
 }
 
 }  // namespace slab
@@ -394,11 +443,24 @@ extern "C" int slab_router_fused_bwd(const float* logits, const int* idx, const 
   return (int)cudaGetLastError();
 }
 
-extern "C" int slab_ce_fwd_bwd(void* logits, const long* targets, float* loss_sum, int rows, int V, float gscale,
-                               cudaStream_t st) {
+template <bool GRAD>
+static int launch_ce(void* logits, const long* targets, float* loss_sum, int rows, int V, float gscale, cudaStream_t st) {
   if (V % 8) return -100;
   if (rows == 0) return 0;
-  int grid = rows < 148 * 4 ? rows : 148 * 4;
-  ce_fwd_bwd_kernel<<<grid, 512, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
+  // rows of up to 32 K columns leave most of 1024 threads without work: four smaller blocks share the SM
+  if (V > 32768)
+    ce_kernel<512, 2, GRAD><<<2 * (rows < 148 ? rows : 148), 512, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
+  else
+    ce_kernel<256, 1, GRAD><<<rows < 148 * 4 ? rows : 148 * 4, 256, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
   return (int)cudaGetLastError();
+}
+
+extern "C" int slab_ce_fwd_bwd(void* logits, const long* targets, float* loss_sum, int rows, int V, float gscale,
+                               cudaStream_t st) {
+  return launch_ce<true>(logits, targets, loss_sum, rows, V, gscale, st);
+}
+
+// The loss alone: the logits are left as they are.
+extern "C" int slab_ce_fwd(const void* logits, const long* targets, float* loss_sum, int rows, int V, cudaStream_t st) {
+  return launch_ce<false>(const_cast<void*>(logits), targets, loss_sum, rows, V, 0.f, st);
 }

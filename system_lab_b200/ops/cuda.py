@@ -34,6 +34,8 @@ _SIGS = {
     "slab_router_fused_fwd": "ppppiiiiifpfps",
     "slab_router_fused_bwd": "pppppfpiiiiifs",
     "slab_ce_fwd_bwd": "pppiifs",
+    "slab_ce_fwd": "pppiis",
+    "slab_scale_bf16": "plps",
     "slab_quant_tensorwise": "ppppls",
     "slab_grouped_gemm_bf16": "i" + "p" * 5 + "i" * 7 + "pii" + "ps",
     "slab_grouped_gemm_fp8": "p" * 7 + "iiiii" + "ps",
@@ -808,54 +810,89 @@ def causal_attention(q, k, v, scale, window):
 
 
 # ------------------------------------------------------------------------------ linear + cross entropy
+def _graph_is_kept() -> bool:
+    """Inside a backward pass: whether its graph may be run again (``retain_graph``, ``create_graph``)."""
+    probe = getattr(torch._C._autograd, "_get_current_graph_task_keep_graph", None)
+    return True if probe is None else bool(probe())
+
+
+def _saved_tensor_hooks_active() -> bool:
+    probe = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)
+    return True if probe is None else probe(False) is not None
+
+
 class _LinearCE(torch.autograd.Function):
     """loss = mean CE(h @ W^T, targets), chunked over rows: logits of one chunk are produced by the tcgen05 GEMM
     (one segment), turned into their own gradient in place by one kernel, and consumed by the two gradient GEMMs
     (input gradient; weight gradient overwriting on the first chunk, accumulating on later ones) before the next
-    chunk, so at most ``chunk_rows x vocab`` logits exist at a time."""
+    chunk, so at most ``chunk_rows x vocab`` logits exist at a time.  ``grads`` False (nothing will be differentiated):
+    the loss alone.
+
+    The gradients are made in the forward pass for a loss gradient of one; backward multiplies them by the real one.  A
+    backward pass that frees its graph is their last reader and does that in place (a kernel that ends at once when the
+    factor is one); a graph that is kept, or saved through hooks, gets a product of its own."""
 
     @staticmethod
-    def forward(ctx, h, weight, targets, chunk_rows):
+    def forward(ctx, h, weight, targets, chunk_rows, grads=True):
         n, hd = h.shape
         v = weight.shape[0]
         loss_sum = torch.zeros(1, dtype=torch.float32, device=h.device)
-        dh = torch.empty_like(h)
-        need_dw = ctx.needs_input_grad[1]            # a frozen projection (LoRA fine-tuning) needs no weight gradient
-        dw = torch.zeros_like(weight) if need_dw else None
+        # a frozen projection (LoRA fine-tuning) needs no weight gradient
+        need_dh, need_dw = grads and ctx.needs_input_grad[0], grads and ctx.needs_input_grad[1]
         gscale = 1.0 / n
         from . import dense_kernels
-        own = dense_kernels() and hd % 64 == 0 and v % _N_MULTIPLE == 0
-        if own and need_dw:
-            dw = torch.empty_like(weight)            # the first chunk's wgrad overwrites, later chunks accumulate
+        own = dense_kernels() and hd % 64 == 0 and v % _N_MULTIPLE == 0 and n > 0
+        dh = torch.empty_like(h) if need_dh else None
+        dw = None
+        if need_dw:                                  # own kernel: the first chunk's wgrad overwrites, later chunks accumulate
+            dw = torch.empty_like(weight) if own else torch.zeros_like(weight)
         for lo in range(0, n, chunk_rows):
             hi = min(lo + chunk_rows, n)
-            if own:
-                off, cnt = _dense_segments(h.device, hi - lo)
-                hc = h[lo:hi]
-                logits = grouped_gemm_raw(0, hc, weight, off, cnt, v, hd, block_n=256)
-                call("slab_ce_fwd_bwd", logits, targets[lo:hi].contiguous(), loss_sum, hi - lo, v, gscale, stream())
-                grouped_gemm_raw(1, logits, weight, off, cnt, v, hd, out=dh[lo:hi], block_n=_pick_bn(hd))
-                if need_dw:
-                    grouped_gemm_raw(2, logits, hc, off, cnt, v, hd, out=dw, accumulate=lo > 0, block_n=_pick_bn(hd))
+            off, cnt = _dense_segments(h.device, hi - lo)
+            hc = h[lo:hi]
+            logits = grouped_gemm_raw(0, hc, weight, off, cnt, v, hd, block_n=256) if own else hc @ weight.t()
+            if not (need_dh or need_dw):
+                call("slab_ce_fwd", logits, targets[lo:hi].contiguous(), loss_sum, hi - lo, v, stream())
                 continue
-            logits = h[lo:hi] @ weight.t()
             call("slab_ce_fwd_bwd", logits, targets[lo:hi].contiguous(), loss_sum, hi - lo, v, gscale, stream())
-            torch.mm(logits, weight, out=dh[lo:hi])
-            if need_dw:
-                dw.addmm_(logits.t(), h[lo:hi])
-        ctx.save_for_backward(dh, dw)
+            if need_dh and own:
+                grouped_gemm_raw(1, logits, weight, off, cnt, v, hd, out=dh[lo:hi], block_n=_pick_bn(hd))
+            elif need_dh:
+                torch.mm(logits, weight, out=dh[lo:hi])
+            if need_dw and own:
+                grouped_gemm_raw(2, logits, hc, off, cnt, v, hd, out=dw, accumulate=lo > 0, block_n=_pick_bn(hd))
+            elif need_dw:
+                dw.addmm_(logits.t(), hc)
+        ctx.hooked = _saved_tensor_hooks_active()
+        if ctx.hooked:
+            ctx.save_for_backward(dh, dw)
+        else:
+            ctx.made = (dh, dw)
         return (loss_sum / n).squeeze(0)
 
     @staticmethod
     def backward(ctx, g):
-        dh, dw = ctx.saved_tensors
-        return dh * g.to(dh.dtype), (dw * g.to(dw.dtype) if dw is not None else None), None, None
+        if ctx.hooked:
+            dh, dw = ctx.saved_tensors
+        elif ctx.made is None:
+            raise RuntimeError("Trying to backward through the graph a second time: pass retain_graph=True to the first "
+                               "backward")
+        else:
+            dh, dw = ctx.made
+        if ctx.hooked or not g.is_cuda or _graph_is_kept():
+            return tuple(t * g.to(t.dtype) if t is not None else None for t in (dh, dw)) + (None, None, None)
+        ctx.made = None
+        g32 = g.float().contiguous()
+        for t in (dh, dw):
+            if t is not None:
+                call("slab_scale_bf16", t, t.numel(), g32, stream())
+        return dh, dw, None, None, None
 
 
 def linear_cross_entropy(h, weight, targets, chunk_rows: int = 8192):
     if not _bf16(h, weight) or weight.shape[0] % 8:
         return ref.linear_cross_entropy(h, weight, targets)
-    return _LinearCE.apply(h.contiguous(), weight.contiguous(), targets.contiguous(), chunk_rows)
+    return _LinearCE.apply(h.contiguous(), weight.contiguous(), targets.contiguous(), chunk_rows, torch.is_grad_enabled())
 
 
 # ------------------------------------------------------------------------------ quantisation
