@@ -1,0 +1,49 @@
+"""Dispatch on one rank: the token-ordered scatter behind both entry points delivers rows, scales, scalars and flags."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,topk,experts,hidden", [(1, 1, 8, 128), (61, 8, 128, 256), (300, 3, 12, 1152), (257, 2, 4, 7168)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_rows_scales_scalars_and_padding(tokens, topk, experts, hidden, fp8, scaled):
+    from system_lab_b200.moe.fused_dispatch import FusedDispatcher
+    from system_lab_b200.ops import cuda
+    from system_lab_b200.parallel.mesh import single_process_mesh
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    d = FusedDispatcher(single_process_mesh(), experts, topk, hidden, tokens, 128, torch.device("cuda", 0), fp8_payload=fp8)
+    x = torch.randn(tokens, hidden, generator=g, device="cuda").bfloat16()
+    p = torch.rand(tokens, topk, generator=g, device="cuda")
+    scale = torch.rand(tokens, topk, generator=g, device="cuda") + 0.5 if scaled else None
+    idx = torch.rand(tokens, experts, generator=g, device="cuda").topk(topk, -1).indices.int()
+    plan = d.plan(idx)
+    rows = (plan.pair_loc & 0xFFFFFF).long().view(tokens, topk)
+    want = x[:, None, :] if scale is None else (x.float()[:, None, :] * scale[..., None])
+    want = want.expand(tokens, topk, hidden)
+    used = int(plan.meta[0])
+    for ordered in (True, False):
+        buf = d.rows_fp8.view(torch.uint8) if fp8 else d.rows[0].view(torch.int16)
+        buf.fill_(1)
+        d.scalars[0].fill_(-1)
+        if ordered:
+            d.scatter_ordered(plan, x, p, 0, scale_in=scale, fp8=fp8).wait()
+        else:
+            d.wait_rows(0, d.scatter(plan, x, p, 0, scale_in=scale, fp8=fp8))
+        cuda.check_status()
+        if not fp8:
+            assert torch.equal(d.rows[0][rows], want.bfloat16())
+        elif scale is None:
+            q, s = cuda.quant_1x128(x)
+            assert torch.equal(d.rows_fp8.view(torch.uint8)[rows], q.view(torch.uint8)[:, None, :].expand(tokens, topk, hidden))
+            assert torch.equal(d.row_scales[rows], s[:, None, :].expand(tokens, topk, hidden // 128))
+        else:                                        # half an e4m3 step (2^-4), doubled for the kernel's reciprocal
+            got = d.rows_fp8[rows].float() * d.row_scales[rows].repeat_interleave(128, -1)
+            assert bool(((got - want).abs() <= want.abs() * 2 ** -3 + d.row_scales[rows].repeat_interleave(128, -1) * 2 ** -9).all())
+        assert torch.equal(d.scalars[0][rows], p)
+        free = torch.ones(used, dtype=torch.bool, device="cuda")
+        free[rows.reshape(-1)] = False
+        assert not bool(buf[:used][free].any()) and not bool(d.scalars[0][:used][free].any())
+        assert torch.equal(d.origin[rows].long(), torch.arange(tokens * topk, device="cuda").view(tokens, topk))
+        assert not bool(d.chunk_done.any()) and not bool(d.done_counter.any())
