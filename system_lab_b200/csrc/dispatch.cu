@@ -77,14 +77,21 @@ moe_count_kernel(const int* __restrict__ topk_idx, int n_pairs, int E, int* __re
 
 // ---------------------------------------------------------------- publish (one block)
 // block_hist -> block_base (exclusive prefix over blocks), send_counts; store counts to every peer.
+// (one block, latency-bound: 64 blocks x 256 experts 13.6 -> 6.6 us with the loads of a batch in flight together)
+constexpr int PUBLISH_BATCH = 16;
 __global__ void moe_publish_kernel(int* __restrict__ block_hist, int n_blocks, int E, int* __restrict__ send_counts,
                                    PeerTable peers, WsLayout ws, int world, int me, int epoch) {
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     int acc = 0;
-    for (int b = 0; b < n_blocks; ++b) {
-      int c = block_hist[b * E + e];
-      block_hist[b * E + e] = acc;          // becomes block_base
-      acc += c;
+    for (int b0 = 0; b0 < n_blocks; b0 += PUBLISH_BATCH) {     // a batch of loads in flight before its stores
+      int c[PUBLISH_BATCH];
+#pragma unroll
+      for (int i = 0; i < PUBLISH_BATCH; ++i) c[i] = b0 + i < n_blocks ? block_hist[(b0 + i) * E + e] : 0;
+#pragma unroll
+      for (int i = 0; i < PUBLISH_BATCH; ++i) {
+        if (b0 + i < n_blocks) block_hist[(b0 + i) * E + e] = acc;          // becomes block_base
+        acc += c[i];
+      }
     }
     send_counts[e] = acc;
     for (int d = 0; d < world; ++d) {
@@ -198,16 +205,23 @@ __global__ void moe_plan_kernel(PeerTable peers, WsLayout ws, int world, int me,
     before[e] = b;
   }
   __syncthreads();
-  if (threadIdx.x < world) {             // one thread per owner rank: aligned prefix over its experts
-    int d = threadIdx.x, acc = 0;
-    for (int j = 0; j < e_local; ++j) {
-      int e = d * e_local + j;
-      seg_off[e] = acc;
-      acc += (total[e] + pad - 1) / pad * pad;
+  // aligned prefix over every owner's experts: one scan over all, less the owner's start (a serial walk of 256 experts by one
+  // thread took most of the kernel's 20 us, 4.9 now)
+  {
+    int all;
+    const int e = threadIdx.x;           // blockDim.x >= E (512 threads, E <= 512)
+    const int pre = block_exclusive_scan(e < E ? (total[e] + pad - 1) / pad * pad : 0, scan_tmp, &all);
+    if (e < E) seg_off[e] = pre;
+    __syncthreads();
+    const int start = e < E ? seg_off[e / e_local * e_local] : 0;
+    if (e < world) {
+      const int acc = (e + 1 < world ? seg_off[(e + 1) * e_local] : all) - seg_off[e * e_local];
+      if (acc > capacity) atomicCAS(status, 0, ST_CAPACITY);
+      if (e == me) meta[0] = acc;
+      atomicMax(&max_rows, acc);
     }
-    if (acc > capacity) atomicCAS(status, 0, ST_CAPACITY);
-    if (d == me) meta[0] = acc;
-    atomicMax(&max_rows, acc);
+    __syncthreads();
+    if (e < E) seg_off[e] = pre - start;
   }
   __syncthreads();
   // the same number on every rank (all of them see all counts): lets the ranks take the same decision about anything

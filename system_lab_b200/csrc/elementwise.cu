@@ -7,6 +7,9 @@
 // (notes/2026-04/2026-04-24_gptoss_17_fused_residual_rmsnorm_impl.md:43-83), SwiGLU*probs forward and
 // no-cat backward (notes/2026-04/2026-04-25_gptoss_23_swiglu_nocat_triton_verify.md:92-113).
 #include <cstdio>
+#include <type_traits>
+
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "slab_noalloc.h"
@@ -650,7 +653,6 @@ __global__ void sumsq_kernel(const G* __restrict__ g, long n, float scale, float
 }
 
 // ------------------------------------------------------------------ flat AdamW
-// One thread handles 4 consecutive elements; a 128-element block (one fp8 scale) is one warp.
 // P: master/weight dtype (float or bf16).  State kinds: 0 fp32, 1 bf16, 2 fp8 (e4m3 + per-128 fp32
 // scale; v is stored as sqrt(v)).  `coef` is the clip coefficient on the device (no host sync).
 struct AdamArgs {
@@ -659,9 +661,123 @@ struct AdamArgs {
                        // packed at the tail of a flat group on 128-element boundaries) do not
 };
 
-// 16 consecutive elements per thread (16-byte accesses for every storage type); the 8 threads that share a
-// 128-element scale block are neighbouring lanes.  If `sq_out` is given the kernel also adds sum(g^2) of the
-// raw gradient to it (the global-norm accumulation of the optimizer-in-backward mode).
+// Bound by memory.  fp32 and bf16 states: a thread owns 8 consecutive elements at a time, so that a warp's 16-byte accesses
+// lie side by side, ADAM_U such pieces 256 elements apart in flight (268 M elements, of 16 consecutive ones per thread
+// before: fp32 1682 -> 1260 us, 5.97 TB/s; bf16 993 -> 731 us, 5.14 TB/s).  If `sq_out` is given the kernel also adds
+// sum(g^2) of the raw gradient to it (the global-norm accumulation of the optimizer-in-backward mode).
+constexpr int ADAM_U = 2;
+
+template <typename T>
+__device__ __forceinline__ void load8(const T* base, long u, float (&f)[8]);
+template <>
+__device__ __forceinline__ void load8<float>(const float* base, long u, float (&f)[8]) {
+  const float4* p = reinterpret_cast<const float4*>(base) + 2 * u;
+  const float4 a = p[0], b = p[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+  f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+template <>
+__device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* base, long u, float (&f)[8]) {
+  unpack8(reinterpret_cast<const bf16x8*>(base)[u], f);
+}
+template <typename T>
+__device__ __forceinline__ void store8(T* base, long u, const float (&f)[8]);
+template <>
+__device__ __forceinline__ void store8<float>(float* base, long u, const float (&f)[8]) {
+  float4* p = reinterpret_cast<float4*>(base) + 2 * u;
+  p[0] = make_float4(f[0], f[1], f[2], f[3]);
+  p[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+template <>
+__device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* base, long u, const float (&f)[8]) {
+  reinterpret_cast<bf16x8*>(base)[u] = pack8(f);
+}
+
+template <typename P, int KIND, typename G>
+__global__ void __launch_bounds__(256)
+adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_raw, void* __restrict__ v_raw,
+             __nv_bfloat16* __restrict__ out_bf16, const float* __restrict__ coef, float* __restrict__ sq_out, long q_begin, long nq, AdamArgs a) {
+  using S = std::conditional_t<KIND == 0, float, __nv_bfloat16>;
+  S* const ms = reinterpret_cast<S*>(m_raw);
+  S* const vs = reinterpret_cast<S*>(v_raw);
+  // One launch covers the 16-element items [q_begin, nq), q_begin a multiple of 32: the 8-element pieces [2 q_begin, 2 nq).
+  __shared__ float red[32];
+  const float c = coef ? *coef : 1.f;
+  const float r1 = 1.f / a.bc1, r2 = rsqrtf(a.bc2);
+  float sq = 0.f;
+  const int lane = threadIdx.x & 31;
+  const long nu = 2 * nq;
+  for (long w0 = 2 * q_begin + (blockIdx.x * (long)blockDim.x + (threadIdx.x & ~31)) * ADAM_U; w0 < nu;
+       w0 += (long)gridDim.x * blockDim.x * ADAM_U) {
+    float gv[ADAM_U][8], mv[ADAM_U][8], vv[ADAM_U][8], pv[ADAM_U][8];
+#pragma unroll
+    for (int h = 0; h < ADAM_U; ++h) {
+      const long u = w0 + h * 32 + lane;
+      if (u < nu) {
+        load8<G>(g, u, gv[h]);
+        load8<P>(p, u, pv[h]);
+        load8<S>(ms, u, mv[h]);
+        load8<S>(vs, u, vv[h]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gv[h][j] = pv[h][j] = mv[h][j] = vv[h][j] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < ADAM_U; ++h) {
+      const long u = w0 + h * 32 + lane;
+      const float decay = (u << 3) < a.decay_end ? 1.f - a.lr * a.wd : 1.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float gr = gv[h][j];
+        sq += gr * gr;
+        const float gj = gr * c;
+        float mo = mv[h][j], vo = vv[h][j];
+        if (KIND != 0) vo *= vo;                    // stored in the sqrt domain
+        mo = a.beta1 * mo + (1.f - a.beta1) * gj;
+        vo = a.beta2 * vo + (1.f - a.beta2) * gj * gj;
+        const float root = sqrtf(vo);
+        pv[h][j] = pv[h][j] * decay - a.lr * (mo * r1) / (root * r2 + a.eps);
+        if (KIND != 0) vo = root;
+        mv[h][j] = mo;
+        vv[h][j] = vo;
+      }
+      if (u < nu) {
+        store8<P>(p, u, pv[h]);
+        if (out_bf16) store8<__nv_bfloat16>(out_bf16, u, pv[h]);
+        store8<S>(ms, u, mv[h]);
+        store8<S>(vs, u, vv[h]);
+      }
+    }
+  }
+  if (sq_out) {
+    sq = block_sum(sq, red);
+    if (threadIdx.x == 0) atomicAdd(sq_out, sq);
+  }
+}
+
+// 8-bit states: 16 consecutive elements per thread, so that a moment is one 16-byte access and 8 neighbouring lanes share a
+// scale block (pieces of 8 as above: 574 -> 745 us).  Its conversions and special functions share a pipe of 16 lanes per
+// clock: two elements per conversion, and the root that is stored also serves the update.
+__device__ __forceinline__ void from_e4m3x16(const uint4& q, float (&f)[16]) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)((k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu),
+                                                     __NV_E4M3);
+    const float2 t = __half22float2(__half2(h));
+    f[2 * k] = t.x;
+    f[2 * k + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 to_e4m3x16(const float (&f)[16]) {
+  float a[8], b[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { a[j] = f[j]; b[j] = f[8 + j]; }
+  const uint2 lo = to_e4m3x8(a), hi = to_e4m3x8(b);
+  return make_uint4(lo.x, lo.y, hi.x, hi.y);
+}
+
 template <typename T>
 __device__ __forceinline__ void load16(const T* base, long i, float (&f)[16]);
 template <>
@@ -700,21 +816,21 @@ __device__ __forceinline__ void store16<__nv_bfloat16>(__nv_bfloat16* base, long
   p[1] = pack8(b);
 }
 
-template <typename P, int KIND, typename G>
+template <typename P, typename G>
 __global__ void __launch_bounds__(256)
-adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_raw, void* __restrict__ v_raw,
+adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_raw, void* __restrict__ v_raw,
              float* __restrict__ m_scale, float* __restrict__ v_scale, __nv_bfloat16* __restrict__ out_bf16,
-             const float* __restrict__ coef, float* __restrict__ sq_out, long q_begin, long nq, AdamArgs a) {
+              const float* __restrict__ coef, float* __restrict__ sq_out, long q_begin, long nq, AdamArgs a) {
   // One launch covers the 16-element items [q_begin, nq); q_begin is a multiple of 32.
   __shared__ float red[32];
   const float c = coef ? *coef : 1.f;
+  const float r1 = 1.f / a.bc1, r2 = rsqrtf(a.bc2);
   float sq = 0.f;
   // warp-uniform trip count: lanes past the end idle through the body so the block-scale shuffles stay full-warp
   for (long i0 = q_begin + blockIdx.x * (long)blockDim.x + (threadIdx.x & ~31); i0 < nq;
        i0 += (long)gridDim.x * blockDim.x) {
     const long i = i0 + (threadIdx.x & 31);
     const bool act = i < nq;
-    if (!act && KIND != 2) continue;
     if (!act) {                                  // nq is a multiple of 8, so whole 8-lane groups are idle together
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) {
@@ -733,69 +849,43 @@ adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_ra
       sq += gv[j] * gv[j];
       gv[j] *= c;
     }
-    if (KIND == 0) {
-      load16<float>(reinterpret_cast<const float*>(m_raw), i, mv);
-      load16<float>(reinterpret_cast<const float*>(v_raw), i, vv);
-    } else if (KIND == 1) {
-      load16<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(m_raw), i, mv);
-      load16<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(v_raw), i, vv);
+    const float ms = m_scale[e0 >> 7], vs = v_scale[e0 >> 7];
+    from_e4m3x16(reinterpret_cast<const uint4*>(m_raw)[i], mv);
+    from_e4m3x16(reinterpret_cast<const uint4*>(v_raw)[i], vv);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) vv[j] *= vv[j];
-    } else {
-      const float ms = m_scale[e0 >> 7], vs = v_scale[e0 >> 7];
-      uint4 mq = reinterpret_cast<const uint4*>(m_raw)[i], vq = reinterpret_cast<const uint4*>(v_raw)[i];
-      const __nv_fp8_e4m3* m8 = reinterpret_cast<const __nv_fp8_e4m3*>(&mq);
-      const __nv_fp8_e4m3* v8 = reinterpret_cast<const __nv_fp8_e4m3*>(&vq);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        mv[j] = float(m8[j]) * ms;
-        float sv = float(v8[j]) * vs;
-        vv[j] = sv * sv;
-      }
+    for (int j = 0; j < 16; ++j) {
+      mv[j] *= ms;
+      const float sv = vv[j] * vs;
+      vv[j] = sv * sv;
     }
     float m_amax = 0.f, v_amax = 0.f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       mv[j] = a.beta1 * mv[j] + (1.f - a.beta1) * gv[j];
       vv[j] = a.beta2 * vv[j] + (1.f - a.beta2) * gv[j] * gv[j];
-      const float denom = sqrtf(vv[j] / a.bc2) + a.eps;
-      pv[j] = pv[j] * decay - a.lr * (mv[j] / a.bc1) / denom;
-      if (KIND != 0) vv[j] = sqrtf(vv[j]);        // stored in the sqrt domain
+      vv[j] = sqrtf(vv[j]);                       // stored in the sqrt domain
+      pv[j] = pv[j] * decay - a.lr * (mv[j] * r1) / (vv[j] * r2 + a.eps);
       m_amax = fmaxf(m_amax, fabsf(mv[j]));
       v_amax = fmaxf(v_amax, vv[j]);
     }
     store16<P>(p, i, pv);
     if (out_bf16) store16<__nv_bfloat16>(out_bf16, i, pv);
-    if (KIND == 0) {
-      store16<float>(reinterpret_cast<float*>(m_raw), i, mv);
-      store16<float>(reinterpret_cast<float*>(v_raw), i, vv);
-    } else if (KIND == 1) {
-      store16<__nv_bfloat16>(reinterpret_cast<__nv_bfloat16*>(m_raw), i, mv);
-      store16<__nv_bfloat16>(reinterpret_cast<__nv_bfloat16*>(v_raw), i, vv);
-    } else {
-      // 8 neighbouring lanes cover one 128-element scale block
+    // 8 neighbouring lanes cover one 128-element scale block
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        m_amax = fmaxf(m_amax, __shfl_xor_sync(0xffffffffu, m_amax, o));
-        v_amax = fmaxf(v_amax, __shfl_xor_sync(0xffffffffu, v_amax, o));
-      }
-      m_amax = fmaxf(m_amax, 1e-30f);
-      v_amax = fmaxf(v_amax, 1e-30f);
-      const float mi = 448.f / m_amax, vi = 448.f / v_amax;
-      uint4 mo, vo;
-      __nv_fp8_e4m3* m8 = reinterpret_cast<__nv_fp8_e4m3*>(&mo);
-      __nv_fp8_e4m3* v8 = reinterpret_cast<__nv_fp8_e4m3*>(&vo);
+    for (int o = 4; o > 0; o >>= 1) {
+      m_amax = fmaxf(m_amax, __shfl_xor_sync(0xffffffffu, m_amax, o));
+      v_amax = fmaxf(v_amax, __shfl_xor_sync(0xffffffffu, v_amax, o));
+    }
+    m_amax = fmaxf(m_amax, 1e-30f);
+    v_amax = fmaxf(v_amax, 1e-30f);
+    const float mi = 448.f / m_amax, vi = 448.f / v_amax;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        m8[j] = __nv_fp8_e4m3(mv[j] * mi);
-        v8[j] = __nv_fp8_e4m3(vv[j] * vi);
-      }
-      reinterpret_cast<uint4*>(m_raw)[i] = mo;
-      reinterpret_cast<uint4*>(v_raw)[i] = vo;
-      if ((threadIdx.x & 7) == 0) {
-        m_scale[e0 >> 7] = m_amax / 448.f;
-        v_scale[e0 >> 7] = v_amax / 448.f;
-      }
+    for (int j = 0; j < 16; ++j) { mv[j] *= mi; vv[j] *= vi; }
+    reinterpret_cast<uint4*>(m_raw)[i] = to_e4m3x16(mv);
+    reinterpret_cast<uint4*>(v_raw)[i] = to_e4m3x16(vv);
+    if ((threadIdx.x & 7) == 0) {
+      m_scale[e0 >> 7] = m_amax / 448.f;
+      v_scale[e0 >> 7] = v_amax / 448.f;
     }
   }
   if (sq_out) {
@@ -1034,11 +1124,11 @@ static void launch_adamw(void* p, const void* g, void* m, void* v, float* m_scal
     const long q1 = q0 + piece < nq ? q0 + piece : nq;
     const int grid = grid_for(q1 - q0, 256, background ? ctas_per_sm : 8);
     if (state_kind == 0)
-      adamw_kernel<P, 0, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, m_scale, v_scale, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
+      adamw_kernel<P, 0, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
     else if (state_kind == 1)
-      adamw_kernel<P, 1, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, m_scale, v_scale, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
+      adamw_kernel<P, 1, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
     else
-      adamw_kernel<P, 2, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, m_scale, v_scale, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
+      adamw8_kernel<P, G><<<grid, 256, 0, st>>>((P*)p, (const G*)g, m, v, m_scale, v_scale, (__nv_bfloat16*)out_bf16, coef, sq_out, q0, q1, a);
   }
 }
 
