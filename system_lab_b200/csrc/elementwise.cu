@@ -757,8 +757,10 @@ adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_ra
 }
 
 // 8-bit states: 16 consecutive elements per thread, so that a moment is one 16-byte access and 8 neighbouring lanes share a
-// scale block (pieces of 8 as above: 574 -> 745 us).  Its conversions and special functions share a pipe of 16 lanes per
-// clock: two elements per conversion, and the root that is stored also serves the update.
+// scale block (pieces of 8 as above: 574 -> 745 us).  Conversions and special functions share a pipe of 16 lanes per clock:
+// with bf16 weights two elements share every conversion, the root that is stored also serves the update, and three blocks
+// fit an SM (268 M elements: 574 -> 556 us, beside other kernels with two blocks per SM 709 -> 632).  fp32 weights are
+// bound by their own traffic and lose by it (845 -> 911 us): element by element there (836).
 __device__ __forceinline__ void from_e4m3x16(const uint4& q, float (&f)[16]) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -817,10 +819,11 @@ __device__ __forceinline__ void store16<__nv_bfloat16>(__nv_bfloat16* base, long
 }
 
 template <typename P, typename G>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(P) == 2 ? 3 : 2)
 adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_raw, void* __restrict__ v_raw,
-             float* __restrict__ m_scale, float* __restrict__ v_scale, __nv_bfloat16* __restrict__ out_bf16,
+              float* __restrict__ m_scale, float* __restrict__ v_scale, __nv_bfloat16* __restrict__ out_bf16,
               const float* __restrict__ coef, float* __restrict__ sq_out, long q_begin, long nq, AdamArgs a) {
+  constexpr bool PAIRED = sizeof(P) == 2;
   // One launch covers the 16-element items [q_begin, nq); q_begin is a multiple of 32.
   __shared__ float red[32];
   const float c = coef ? *coef : 1.f;
@@ -850,8 +853,17 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
       gv[j] *= c;
     }
     const float ms = m_scale[e0 >> 7], vs = v_scale[e0 >> 7];
-    from_e4m3x16(reinterpret_cast<const uint4*>(m_raw)[i], mv);
-    from_e4m3x16(reinterpret_cast<const uint4*>(v_raw)[i], vv);
+    const uint4 mq = reinterpret_cast<const uint4*>(m_raw)[i], vq = reinterpret_cast<const uint4*>(v_raw)[i];
+    if (PAIRED) {
+      from_e4m3x16(mq, mv);
+      from_e4m3x16(vq, vv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        mv[j] = float(reinterpret_cast<const __nv_fp8_e4m3*>(&mq)[j]);
+        vv[j] = float(reinterpret_cast<const __nv_fp8_e4m3*>(&vq)[j]);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       mv[j] *= ms;
@@ -863,8 +875,10 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
     for (int j = 0; j < 16; ++j) {
       mv[j] = a.beta1 * mv[j] + (1.f - a.beta1) * gv[j];
       vv[j] = a.beta2 * vv[j] + (1.f - a.beta2) * gv[j] * gv[j];
-      vv[j] = sqrtf(vv[j]);                       // stored in the sqrt domain
-      pv[j] = pv[j] * decay - a.lr * (mv[j] * r1) / (vv[j] * r2 + a.eps);
+      const float root = sqrtf(vv[j]);            // stored in the sqrt domain
+      const float denom = (PAIRED ? root * r2 : sqrtf(vv[j] / a.bc2)) + a.eps;
+      pv[j] = pv[j] * decay - a.lr * (PAIRED ? mv[j] * r1 : mv[j] / a.bc1) / denom;
+      vv[j] = root;
       m_amax = fmaxf(m_amax, fabsf(mv[j]));
       v_amax = fmaxf(v_amax, vv[j]);
     }
@@ -881,8 +895,19 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
     const float mi = 448.f / m_amax, vi = 448.f / v_amax;
 #pragma unroll
     for (int j = 0; j < 16; ++j) { mv[j] *= mi; vv[j] *= vi; }
-    reinterpret_cast<uint4*>(m_raw)[i] = to_e4m3x16(mv);
-    reinterpret_cast<uint4*>(v_raw)[i] = to_e4m3x16(vv);
+    if (PAIRED) {
+      reinterpret_cast<uint4*>(m_raw)[i] = to_e4m3x16(mv);
+      reinterpret_cast<uint4*>(v_raw)[i] = to_e4m3x16(vv);
+    } else {
+      uint4 mo, vo;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        reinterpret_cast<__nv_fp8_e4m3*>(&mo)[j] = __nv_fp8_e4m3(mv[j]);
+        reinterpret_cast<__nv_fp8_e4m3*>(&vo)[j] = __nv_fp8_e4m3(vv[j]);
+      }
+      reinterpret_cast<uint4*>(m_raw)[i] = mo;
+      reinterpret_cast<uint4*>(v_raw)[i] = vo;
+    }
     if ((threadIdx.x & 7) == 0) {
       m_scale[e0 >> 7] = m_amax / 448.f;
       v_scale[e0 >> 7] = v_amax / 448.f;
