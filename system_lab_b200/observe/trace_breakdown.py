@@ -29,9 +29,10 @@ RULES: list[tuple[str, tuple[str, ...]]] = [
     ("slab_norm", ("rmsnorm_fwd_kernel", "rmsnorm_bwd_kernel", "colsum_to_bf16")),
     ("slab_act", ("swiglu_fwd_kernel", "swiglu_bwd_kernel", "rope_kernel")),
     ("slab_router", ("router_topk_kernel",)),
-    ("slab_ce", ("ce_fwd_bwd_kernel",)),
-    ("slab_quant", ("quant_1x128_kernel", "quant_128x128_kernel", "quant_rowwise_kernel")),
-    ("slab_optimizer", ("adamw_kernel", "sumsq_kernel")),
+    ("slab_ce", ("slab::ce_kernel", "ce_fwd_bwd_kernel", "scale_bf16_kernel")),
+    ("slab_quant", ("quant_1x128_kernel", "quant_128x128_kernel", "quant_rowwise_kernel", "quant_rowwise_long",
+                    "quant_tensorwise_kernel", "amax_bf16_kernel")),
+    ("slab_optimizer", ("adamw_kernel", "adamw8_kernel", "sumsq_kernel")),
     ("slab_attn", ("slab_attn", "attn_fwd_kernel", "attn_bwd_kernel")),
     ("slab_fsdp", ("fsdp_gather_kernel", "fsdp_reduce_scatter_kernel", "fsdp_stage_kernel", "fsdp_rs_adamw")),
     ("nccl_rs", ()), ("nccl_ar", ()), ("nccl_ag", ()), ("nccl_a2a", ()), ("nccl_bcast", ()), ("nccl_generic", ()),
