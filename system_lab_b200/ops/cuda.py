@@ -816,6 +816,12 @@ def _graph_is_kept() -> bool:
     return True if probe is None else bool(probe())
 
 
+def _plain_tensor(g) -> bool:
+    """Storage of its own that a kernel can be given: not a tensor subclass, not one of vmap's (``is_grads_batched``)."""
+    fn = torch._C._functorch
+    return type(g) is torch.Tensor and not fn.is_functorch_wrapped_tensor(g) and not fn.is_legacy_batchedtensor(g)
+
+
 def _saved_tensor_hooks_active() -> bool:
     probe = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)
     return True if probe is None else probe(False) is not None
@@ -830,7 +836,8 @@ class _LinearCE(torch.autograd.Function):
 
     The gradients are made in the forward pass for a loss gradient of one; backward multiplies them by the real one.  A
     backward pass that frees its graph is their last reader and does that in place (a kernel that ends at once when the
-    factor is one); a graph that is kept, or saved through hooks, gets a product of its own."""
+    factor is one); a graph that is kept, or saved through hooks, gets a product of its own, and so does a gradient that
+    is itself differentiated (``create_graph``, with or without ``retain_graph``) or comes as a batch."""
 
     @staticmethod
     def forward(ctx, h, weight, targets, chunk_rows, grads=True):
@@ -879,7 +886,7 @@ class _LinearCE(torch.autograd.Function):
                                "backward")
         else:
             dh, dw = ctx.made
-        if ctx.hooked or not g.is_cuda or _graph_is_kept():
+        if ctx.hooked or not g.is_cuda or torch.is_grad_enabled() or _graph_is_kept() or not _plain_tensor(g):
             return tuple(t * g.to(t.dtype) if t is not None else None for t in (dh, dw)) + (None, None, None)
         ctx.made = None
         g32 = g.float().contiguous()

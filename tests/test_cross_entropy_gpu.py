@@ -67,6 +67,23 @@ def test_head_gradients_by_every_route(factor, chunk):
         torch.autograd.grad(once, [x])
 
 
+def test_head_gradients_that_are_differentiated_or_come_as_a_batch():
+    from system_lab_b200.ops import cuda
+    x, w, t = _head(130, 128, 320)
+    f = torch.tensor(0.5, device="cuda", requires_grad=True)             # scaling a gradient by it is exact in bf16
+    dx, dw = torch.autograd.grad(cuda.linear_cross_entropy(x, w, t), [x, w])
+    sx, sw = torch.autograd.grad(cuda.linear_cross_entropy(x, w, t) * f, [x, w], create_graph=True, retain_graph=False)
+    assert torch.equal(sx.detach(), dx * 0.5) and torch.equal(sw.detach(), dw * 0.5)
+    (df,) = torch.autograd.grad(sx.double().sum() + sw.double().sum(), f)
+    want = float(dx.double().sum() + dw.double().sum())
+    # the sums over the two gradients are rounded to bf16 (2^-9 each)
+    assert abs(float(df) - want) <= 2 ** -8 * float(dx.double().sum().abs() + dw.double().sum().abs())
+    bx, bw = torch.autograd.grad(cuda.linear_cross_entropy(x, w, t), [x, w], torch.tensor([1.0, 2.0], device="cuda"),
+                                 is_grads_batched=True)
+    for got, one in ((bx, dx), (bw, dw)):
+        assert torch.equal(got[0], one) and torch.equal(got[1], one * 2)
+
+
 def test_head_without_gradients_is_the_same_loss():
     from system_lab_b200.ops import cuda
     x, w, t = _head(200, 128, 320)
