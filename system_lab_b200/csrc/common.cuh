@@ -100,6 +100,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
   }
 }
+// The same answer in all lanes of a converged warp.  Lanes that poll on their own may disagree when a barrier completes
+// just as another role gives up, and a warp that is split then never meets again at what follows (.aligned instructions,
+// named barriers).  Epilogue warps that share named barriers remember the answer and, once it is no, walk the rest of their
+// tiles without waiting or storing, so that every barrier still has all its threads.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
 
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {

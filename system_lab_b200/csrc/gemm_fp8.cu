@@ -135,7 +135,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       f8_get_tile(t, prefix, p, ti);
       const int a_row = warp_uniform(ti.row0), b_row = warp_uniform(ti.e * p.N + ti.n_idx * F8_BN);
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY));
+        ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
         if (!ok) break;
         uint8_t* a_dst = ring + s * F8_STAGE;
         if (elect_one()) {
@@ -185,8 +185,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     uint8_t* sbuf = store_buf + half * F8_STORE_BYTES;
     uint32_t it = 0;
     F8Tile ti;
-    bool ok = true;
-    for (int t = blockIdx.x; ok && f8_get_tile(t, prefix, p, ti); t += gridDim.x) {
+    bool ok = true;                                      // no wait of this warp has run out (see mbar_wait_warp)
+    for (int t = blockIdx.x; f8_get_tile(t, prefix, p, ti); t += gridDim.x) {
       unsigned long long acc[32];                        // two fp32 columns each
 #pragma unroll
       for (int i = 0; i < 32; ++i) acc[i] = 0ull;
@@ -201,13 +201,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       float sc[F8_AHEAD];
 #pragma unroll
       for (int i = 0; i < F8_AHEAD; ++i) sc[i] = scale_at(i);
-      for (int kb = 0; kb < kblocks; ++kb, ++it) {
+      for (int kb = 0; ok && kb < kblocks; ++kb, ++it) {
         const uint32_t buf = it % F8_TBUF;
         const float now = sc[0];
 #pragma unroll
         for (int i = 0; i + 1 < F8_AHEAD; ++i) sc[i] = sc[i + 1];
         sc[F8_AHEAD - 1] = scale_at(kb + F8_AHEAD);
-        if (!mbar_wait(&tfull_bar[buf], (it / F8_TBUF) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        ok = mbar_wait_warp(&tfull_bar[buf], (it / F8_TBUF) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * F8_BN + half * 64;
         uint32_t v0[32], v1[32];
@@ -224,7 +225,6 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
           acc[16 + i] = fma_f32x2(f32x2(v1[2 * i], v1[2 * i + 1]), s2, acc[16 + i]);
         }
       }
-      if (!ok) break;
       // this group's 64 columns: swizzled staging (one buffer per group) -> TMA store
       if (store_thread) tma_store_wait_read<0>();
       if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
@@ -240,7 +240,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       }
       fence_proxy_async();
       if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
-      if (store_thread) {
+      if (ok && store_thread) {
         tma_store_2d(&tmap_c, sbuf, ti.n_idx * F8_BN + half * 64, ti.row0);
         tma_store_commit();
       }

@@ -374,7 +374,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       const int x0 = MODE == PG_WGRAD ? ti.cb * p.width + (int)cta * half : ti.row0 + (int)cta * half;
       const CUtensorMap* x_map = &maps.x[X_MN ? (half == 128 ? 3 : 2) : units - 1];
       for (int ks = 0; ks < ti.ksteps; ++ks) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY));
+        ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
         if (!ok) break;
         const uint32_t w_dst = ring_addr + s * PG_STAGE, x_dst = w_dst + PG_OPERAND, bar = bar0 + s * 8;
         if (elect_one()) {
@@ -412,14 +412,14 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         pg_uniform(ti);
         if (ti.ksteps == 0) continue;
         const int buf = it & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY));
+        ok = mbar_wait_warp(&tempty_bar[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d = tmem_base + buf * 256;
         const uint32_t idesc = make_idesc(FP8 ? 0 : 1, FP8 ? 0 : 1, W_MN ? 1 : 0, X_MN ? 1 : 0, 256, ti.n);
         int left = ti.mmas;
         for (int ks = 0; ks < ti.ksteps; ++ks) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, abort_flag, p.status, ST_TIMEOUT_FULL));
+          ok = mbar_wait_warp(&full_bar[s], ph, abort_flag, p.status, ST_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
           const uint64_t wd = wd0 + (uint32_t)(s * (PG_STAGE >> 4)), xd = xd0 + (uint32_t)(s * (PG_STAGE >> 4));
@@ -446,6 +446,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
     uint64_t* const old_g = old_bar + 2 * grp;
     int it = 0, ctr = 0;
     int slot = 0;                                 // FWD / DGRAD: staging buffer in turn
+    bool ok = true;                               // no wait of this warp has run out (see mbar_wait_warp)
     PairTile ti;
     ti.e = 0;
     for (int t = pair; t < tiles; t += pairs) {
@@ -458,7 +459,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       // goes through guarded global accesses.  All others leave by TMA, and a sum onto the old result has that brought in
       // by TMA as well (a thread's own row is a line per access when read from global memory), one chunk ahead.
       const bool hangs = MODE == PG_WGRAD && m0 + 128 > p.N;
-      if (MODE == PG_WGRAD && p.accumulate && !empty && !hangs && store_thread) {
+      if (MODE == PG_WGRAD && p.accumulate && !empty && !hangs && ok && store_thread) {
         if (ti.cb * ti.width + grp * 64 < p.K && grp * 64 < ti.width) {
           tma_store_wait_read<0>();
           mbar_arrive_expect_tx(&old_g[ctr & 1], 16384);
@@ -478,7 +479,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         sa_next = r < p.R ? __ldg(p.sa + r) : 0.f;
       }
       if (!empty) {
-        if (!mbar_wait(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) break;
+        ok = ok && mbar_wait_warp(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
         tc_fence_after();
       }
       if (MODE != PG_WGRAD) {
@@ -538,7 +539,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           // three buffers in turn: all but the last store have been read, so the next buffer is free
           if (store_thread) tma_store_wait_read<1>();
           pg_group_sync(grp);
-          if (store_thread) {
+          if (ok && store_thread) {
             const uint8_t* b = stage + slot * L::STORE_BUF;
             if (m0 < out_cols && row < p.R) tma_store_2d(&maps.c, b, m0, row);
             if (m0 + 64 < out_cols && row < p.R) tma_store_2d(&maps.c, b + 4096, m0 + 64, row);
@@ -557,7 +558,6 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         const bool row_ok = m0 + r_in_tile < p.N;
         __nv_bfloat16* c_row = p.C + ((size_t)ti.e * p.N + m0 + r_in_tile) * p.K;
         const int chunks = (empty && p.accumulate) ? 0 : min(ti.width, p.K - col0) >> 6;
-        bool ok = true;
 #pragma unroll 1
         for (int c = grp; c < chunks; c += 2) {
           uint32_t lo[32], hi[32];
@@ -570,7 +570,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
             for (int i = 0; i < 32; ++i) lo[i] = hi[i] = 0u;
           }
           if (hangs) {
-            if (row_ok) {
+            if (ok && row_ok) {
 #pragma unroll
               for (int g = 0; g < 8; ++g) {
                 const uint32_t* v = g < 4 ? lo + g * 8 : hi + (g - 4) * 8;
@@ -590,9 +590,8 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           }
           uint8_t* sbuf = stage + (ctr & 1) * 16384;
           if (p.accumulate) {
-            ok = mbar_wait(&old_g[ctr & 1], (ctr >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
-            if (!ok) break;
-            if (store_thread && c + 2 < chunks) {   // the group's next chunk, into the buffer whose store came before this one
+            ok = ok && mbar_wait_warp(&old_g[ctr & 1], (ctr >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
+            if (ok && store_thread && c + 2 < chunks) {   // the group's next chunk, into the buffer whose store came before this one
               tma_store_wait_read<0>();
               mbar_arrive_expect_tx(&old_g[(ctr + 1) & 1], 16384);
               tma_load_2d(stage + ((ctr + 1) & 1) * 16384, &maps.c, &old_g[(ctr + 1) & 1], col0 + c * 64 + 128,
@@ -618,13 +617,12 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           }
           fence_proxy_async();
           pg_group_sync(grp);
-          if (store_thread) {
+          if (ok && store_thread) {
             tma_store_2d(&maps.c, sbuf, col0 + c * 64, ti.e * p.N + m0);
             tma_store_commit();
           }
           ++ctr;
         }
-        if (!ok) break;
         if (!empty) {
           tc_fence_before();
           __syncwarp();

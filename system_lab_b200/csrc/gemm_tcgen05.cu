@@ -314,6 +314,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     int it = 0;
     int chunk_ctr = 0;                          // staging buffer toggles per 64-column chunk
     int tile_ctr = 0;
+    bool ok = true;                             // no wait of this warp has run out (see mbar_wait_warp)
     TileInfo ti;
     for (int t = blockIdx.x; get_tile<MODE, BN>(t, prefix, p, n_tiles, ti); t += gridDim.x) {
       const int col0 = ti.n_idx * BN;
@@ -328,7 +329,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         ++tile_ctr;
       }
       const int buf = it & 1;
-      if (!mbar_wait(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) break;
+      ok = ok && mbar_wait_warp(&tfull_bar[buf], (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * BN;
 #pragma unroll 1
@@ -363,7 +364,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const int row = idx >> 3, seg = idx & 7;
             const int org = org_tile[row];
             const int col = col0 + c + seg * 8;
-            if (org >= 0 && col < out_cols) {
+            if (ok && org >= 0 && col < out_cols) {
               const int src = org >> 24, pair = org & 0xFFFFFF;
               if (src >= p.world || pair >= p.pairs) {         // corrupt table: report, never write
                 atomicCAS(p.status, 0, ST_BAD_INDEX);
@@ -374,7 +375,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               *reinterpret_cast<uint4*>(dst) = val;
             }
           }
-        } else if (store_thread) {
+        } else if (ok && store_thread) {
           if (col0 + c < out_cols) tma_store_2d(&tmap_c, sb, col0 + c, tile_row);   // a chunk past the last column has nothing to store
           tma_store_commit();
         }

@@ -87,3 +87,42 @@ def test_row_scaled_e4m3(counts, n, k):
         m = (wq[e].double() * sw[e][:, None].double()).t()
         # the tensor core adds e4m3 products with fewer bits than fp32 (2^-13 of the summed magnitudes at most)
         _close(out[o:o + c], x @ m, (x.abs() @ m.abs()) * 2 ** 7)
+
+
+class _Arrived:
+    """Arrival flags as a dispatcher hands them over: the first ``n`` experts' rows are there, the others never come."""
+
+    def __init__(self, n, experts):
+        self.flags = (torch.arange(experts, device="cuda") < n).int().view(1, experts)
+        self.world, self.epoch, self.gemm_max_ctas, self.d = 1, 1, 4, self
+
+    def mark_consumed(self):
+        pass
+
+    join_side = mark_consumed
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("arrived", [0, 1, 5, 11, 12])
+def test_rows_that_never_arrive_end_the_launch(mode, arrived):
+    """The wait for the missing rows runs out (20 ms) while the accumulators of the tiles before them are being read out: the
+    kernel returns with the status code, what it computed until then is right, and the next launch is healthy."""
+    from system_lab_b200.ops import cuda
+    n, k, counts = 320, 192, [300] * 12
+    a, dy, w, off, cnt = _operands(counts, n, k, 5)
+    x = (a, dy)[mode]
+    whole = cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k)
+    out = torch.zeros_like(whole)
+    cuda.register("slab_moe_set_wait_limit_ms", "l")
+    cuda.lib().slab_moe_set_wait_limit_ms(20)
+    try:
+        cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k, out=out, ready=_Arrived(arrived, len(counts)))
+        torch.cuda.synchronize()
+        assert cuda.peek_status() == (0 if arrived == 12 else 5)
+    finally:
+        cuda.lib().slab_moe_set_wait_limit_ms(60000)
+        cuda.clear_status()
+    same = (out == whole) | (out == 0)                       # a tile is stored whole or left alone
+    assert bool(same.all()) and (arrived < 12 or torch.equal(out, whole))
+    assert torch.equal(cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k), whole)
+    cuda.check_status()
