@@ -230,8 +230,11 @@ __global__ void moe_plan_kernel(PeerTable peers, WsLayout ws, int world, int me,
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     send_base[e] = seg_off[e] + before[e];
     if (e / e_local == me) {
-      expert_offsets[e - me * e_local] = seg_off[e];
-      expert_counts[e - me * e_local] = total[e];
+      // rows beyond the buffer were reported above and are dropped by the senders: the segments end with the buffer (a
+      // multiple of `pad`), so that nothing that walks them, alignment rows included, leaves it
+      const int off = min(seg_off[e], capacity);
+      expert_offsets[e - me * e_local] = off;
+      expert_counts[e - me * e_local] = min(total[e], capacity - off);
     }
   }
 }
@@ -834,7 +837,7 @@ extern "C" int slab_moe_plan_slots(const int* topk_idx, int n_pairs, int E, cons
                                    int pad, int capacity, int* expert_offsets, int* expert_counts, int* send_base,
                                    int* meta, int* pair_loc, int* status, const int* send_counts, int* send_prefix,
                                    int* item_prefix, int* perm, cudaStream_t st) {
-  if (E > MAX_EXPERTS || world > MAX_WORLD || capacity >= (1 << 24)) return -100;
+  if (E > MAX_EXPERTS || world > MAX_WORLD || capacity >= (1 << 24) || pad < 1 || capacity % pad) return -100;
   if ((send_prefix == nullptr) != (item_prefix == nullptr) || (send_prefix == nullptr) != (perm == nullptr)) return -101;
   PeerTable pt = make_peers(peer_ptrs, world);
   WsLayout ws = make_layout(ws_offsets);

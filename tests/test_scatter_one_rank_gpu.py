@@ -47,3 +47,33 @@ def test_rows_scales_scalars_and_padding(tokens, topk, experts, hidden, fp8, sca
         assert not bool(buf[:used][free].any()) and not bool(d.scalars[0][:used][free].any())
         assert torch.equal(d.origin[rows].long(), torch.arange(tokens * topk, device="cuda").view(tokens, topk))
         assert not bool(d.chunk_done.any()) and not bool(d.done_counter.any())
+
+
+@pytest.mark.parametrize("ordered", [False, True])
+def test_segments_that_do_not_fit_end_with_the_buffer(ordered):
+    """Two ranks whose tokens all pick rank 0's first two experts, 912 padded rows for a buffer of 640: reported, and neither
+    rows nor alignment rows land outside the receive region."""
+    from system_lab_b200.ops import cuda
+    from tests.test_dispatch_gpu import _make
+    ds = _make(2, 200, 2, 8, 256, factor=0.25)
+    cap = ds[0].capacity
+    idx = torch.tensor([0, 1], device="cuda", dtype=torch.int32).repeat(200, 1)
+    plans = [d.plan_finish(*p) for d, p in zip(ds, [d.plan_publish(idx) for d in ds])]
+    torch.cuda.synchronize()
+    assert cap == 640 and cuda.peek_status() == 7
+    cuda.clear_status()
+    assert plans[0].expert_offsets.tolist() == [0, 512, 640, 640] and plans[0].expert_counts.tolist() == [400, 128, 0, 0]
+    outside = [d.ws.buf[d.off["rows1"]:d.off["origin"]] for d in ds]
+    for o in outside:
+        o.fill_(77)
+    x = torch.ones(200, 256, device="cuda", dtype=torch.bfloat16)
+    for d, plan in zip(ds, plans):
+        if ordered:
+            d.scatter_ordered(plan, x, None, 0)
+        else:
+            d.scatter(plan, x, None, 0)
+    torch.cuda.synchronize()
+    assert all(bool((o[:d.off["scalars0"] - d.off["rows1"]] == 77).all()) for d, o in zip(ds, outside))
+    assert all(bool((o[d.off["out_rows"] - d.off["rows1"]:] == 77).all()) for d, o in zip(ds, outside))
+    assert bool((ds[0].rows[0][:400] == 1).all()) and not bool(ds[0].rows[0][400:512].any())
+    assert bool((ds[0].rows[0][512:640] == 1).all())
