@@ -656,7 +656,8 @@ __global__ void sumsq_kernel(const G* __restrict__ g, long n, float scale, float
 // P: master/weight dtype (float or bf16).  State kinds: 0 fp32, 1 bf16, 2 fp8 (e4m3 + per-128 fp32
 // scale; v is stored as sqrt(v)).  `coef` is the clip coefficient on the device (no host sync).
 struct AdamArgs {
-  float lr, beta1, beta2, eps, wd, bc1, bc2;
+  AdamStep step;
+  float decay;         // 1 - lr * weight decay
   long decay_end;      // elements [0, decay_end) of the shard get weight decay, the rest (norm gains: 1-D parameters,
                        // packed at the tail of a flat group on 128-element boundaries) do not
 };
@@ -703,7 +704,6 @@ adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_ra
   // One launch covers the 16-element items [q_begin, nq), q_begin a multiple of 32: the 8-element pieces [2 q_begin, 2 nq).
   __shared__ float red[32];
   const float c = coef ? *coef : 1.f;
-  const float r1 = 1.f / a.bc1, r2 = rsqrtf(a.bc2);
   float sq = 0.f;
   const int lane = threadIdx.x & 31;
   const long nu = 2 * nq;
@@ -726,21 +726,14 @@ adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_ra
 #pragma unroll
     for (int h = 0; h < ADAM_U; ++h) {
       const long u = w0 + h * 32 + lane;
-      const float decay = (u << 3) < a.decay_end ? 1.f - a.lr * a.wd : 1.f;
+      const float decay = (u << 3) < a.decay_end ? a.decay : 1.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float gr = gv[h][j];
         sq += gr * gr;
-        const float gj = gr * c;
-        float mo = mv[h][j], vo = vv[h][j];
-        if (KIND != 0) vo *= vo;                    // stored in the sqrt domain
-        mo = a.beta1 * mo + (1.f - a.beta1) * gj;
-        vo = a.beta2 * vo + (1.f - a.beta2) * gj * gj;
-        const float root = sqrtf(vo);
-        pv[h][j] = pv[h][j] * decay - a.lr * (mo * r1) / (root * r2 + a.eps);
-        if (KIND != 0) vo = root;
-        mv[h][j] = mo;
-        vv[h][j] = vo;
+        if (KIND != 0) vv[h][j] *= vv[h][j];        // stored in the sqrt domain
+        const float root = adam_step(a.step, decay, gr * c, pv[h][j], mv[h][j], vv[h][j]);
+        if (KIND != 0) vv[h][j] = root;
       }
       if (u < nu) {
         store8<P>(p, u, pv[h]);
@@ -758,9 +751,9 @@ adamw_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_ra
 
 // 8-bit states: 16 consecutive elements per thread, so that a moment is one 16-byte access and 8 neighbouring lanes share a
 // scale block (pieces of 8 as above: 574 -> 745 us).  Conversions and special functions share a pipe of 16 lanes per clock:
-// with bf16 weights two elements share every conversion, the root that is stored also serves the update, and three blocks
-// fit an SM (268 M elements: 574 -> 556 us, beside other kernels with two blocks per SM 709 -> 632).  fp32 weights are
-// bound by their own traffic and lose by it (845 -> 911 us): element by element there (836).
+// with bf16 weights two elements share every conversion and three blocks fit an SM (268 M elements: 574 -> 556 us, beside
+// other kernels with two blocks per SM 709 -> 632).  fp32 weights are bound by their own traffic and lose by paired
+// conversions (845 -> 911 us): element by element there (833).
 __device__ __forceinline__ void from_e4m3x16(const uint4& q, float (&f)[16]) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -827,7 +820,6 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
   // One launch covers the 16-element items [q_begin, nq); q_begin is a multiple of 32.
   __shared__ float red[32];
   const float c = coef ? *coef : 1.f;
-  const float r1 = 1.f / a.bc1, r2 = rsqrtf(a.bc2);
   float sq = 0.f;
   // warp-uniform trip count: lanes past the end idle through the body so the block-scale shuffles stay full-warp
   for (long i0 = q_begin + blockIdx.x * (long)blockDim.x + (threadIdx.x & ~31); i0 < nq;
@@ -843,7 +835,7 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
       continue;
     }
     const long e0 = i << 4;
-    const float decay = e0 < a.decay_end ? 1.f - a.lr * a.wd : 1.f;
+    const float decay = e0 < a.decay_end ? a.decay : 1.f;
     float gv[16], mv[16], vv[16], pv[16];
     load16<G>(g, i, gv);
     load16<P>(p, i, pv);
@@ -873,12 +865,7 @@ adamw8_kernel(P* __restrict__ p, const G* __restrict__ g, void* __restrict__ m_r
     float m_amax = 0.f, v_amax = 0.f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      mv[j] = a.beta1 * mv[j] + (1.f - a.beta1) * gv[j];
-      vv[j] = a.beta2 * vv[j] + (1.f - a.beta2) * gv[j] * gv[j];
-      const float root = sqrtf(vv[j]);            // stored in the sqrt domain
-      const float denom = (PAIRED ? root * r2 : sqrtf(vv[j] / a.bc2)) + a.eps;
-      pv[j] = pv[j] * decay - a.lr * (PAIRED ? mv[j] * r1 : mv[j] / a.bc1) / denom;
-      vv[j] = root;
+      vv[j] = adam_step(a.step, decay, gv[j], pv[j], mv[j], vv[j]);      // stored in the sqrt domain
       m_amax = fmaxf(m_amax, fabsf(mv[j]));
       v_amax = fmaxf(v_amax, vv[j]);
     }
@@ -1169,7 +1156,7 @@ extern "C" int slab_adamw(void* p, int p_is_bf16, const void* g, int g_is_bf16, 
   if (n % 128) return -100;
   if (n == 0) return 0;
   if (decay_end % 128) return -101;
-  AdamArgs a{lr, beta1, beta2, eps, wd, bc1, bc2, decay_end};
+  AdamArgs a{adam_scalars(lr, beta1, beta2, eps, bc1, bc2), 1.f - lr * wd, decay_end};
   if (p_is_bf16) {
     if (g_is_bf16) launch_adamw<__nv_bfloat16, __nv_bfloat16>(p, g, m, v, m_scale, v_scale, out_bf16, coef, sq_out, n, state_kind, a, ctas_per_sm, st);
     else launch_adamw<__nv_bfloat16, float>(p, g, m, v, m_scale, v_scale, out_bf16, coef, sq_out, n, state_kind, a, ctas_per_sm, st);

@@ -136,7 +136,8 @@ fsdp_gather_range_kernel(uint8_t* __restrict__ dst, long lo, long hi, long shard
 }
 
 struct FsAdam {
-  float lr, beta1, beta2, eps, wd, bc1, bc2;
+  AdamStep step;
+  float decay;        // 1 - lr * weight decay
   long decay_end;     // elements [0, decay_end) of the shard get weight decay (the tail holds the 1-D parameters)
 };
 
@@ -195,17 +196,14 @@ fsdp_reduce_scatter_kernel(const uint8_t* __restrict__ mc, float* __restrict__ p
       float4* mm = reinterpret_cast<float4*>(m) + 2 * i;
       float4* vm = reinterpret_cast<float4*>(v) + 2 * i;
       float p8[8], m8[8], v8[8];
-      const float decay = (i << 3) < a.decay_end ? 1.f - a.lr * a.wd : 1.f;
+      const float decay = (i << 3) < a.decay_end ? a.decay : 1.f;
       *reinterpret_cast<float4*>(p8) = pm[0]; *reinterpret_cast<float4*>(p8 + 4) = pm[1];
       *reinterpret_cast<float4*>(m8) = mm[0]; *reinterpret_cast<float4*>(m8 + 4) = mm[1];
       *reinterpret_cast<float4*>(v8) = vm[0]; *reinterpret_cast<float4*>(v8 + 4) = vm[1];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         sq += acc[j] * acc[j];
-        const float g = acc[j] * c;
-        m8[j] = a.beta1 * m8[j] + (1.f - a.beta1) * g;
-        v8[j] = a.beta2 * v8[j] + (1.f - a.beta2) * g * g;
-        p8[j] = p8[j] * decay - a.lr * (m8[j] / a.bc1) / (sqrtf(v8[j] / a.bc2) + a.eps);
+        adam_step(a.step, decay, acc[j] * c, p8[j], m8[j], v8[j]);
       }
       pm[0] = *reinterpret_cast<float4*>(p8); pm[1] = *reinterpret_cast<float4*>(p8 + 4);
       mm[0] = *reinterpret_cast<float4*>(m8); mm[1] = *reinterpret_cast<float4*>(m8 + 4);
@@ -300,7 +298,7 @@ extern "C" int slab_fsdp_reduce_scatter_adamw(long shard_numel, const long* peer
                                               float beta1, float beta2, float eps, float wd, float bc1, float bc2,
                                               long decay_end, int* status, int* done_counter, cudaStream_t st) {
   if (shard_numel % 8 || world > FS_MAX_WORLD || decay_end % 8) return -100;
-  FsAdam a{lr, beta1, beta2, eps, wd, bc1, bc2, decay_end};
+  FsAdam a{adam_scalars(lr, beta1, beta2, eps, bc1, bc2), 1.f - lr * wd, decay_end};
   fsdp_reduce_scatter_kernel<true><<<fs_grid(shard_numel / 8), 512, 0, st>>>(
       fs_multicast(peer_ptrs, world), nullptr, shard_numel / 8, fs_peers(peer_ptrs, world), fs_layout(layout), world, me, slot, epoch, scale, master,
       m, v, (__nv_bfloat16*)out_bf16, coef, sq_out, a, status, g_fs_limit_ns, done_counter);
