@@ -33,9 +33,8 @@
 namespace slab {
 
 constexpr int PG_THREADS = 320;
-constexpr int PG_STAGES = 5;
-constexpr int PG_OPERAND = 128 * 128;            // bytes of one operand in one stage: 128 rows of 128 bytes
-constexpr int PG_STAGE = 2 * PG_OPERAND;
+constexpr int PG_MAX_STAGES = 8;
+constexpr int PG_OPERAND = 128 * 128;            // bytes of a whole operand in one stage: 128 rows of 128 bytes
 constexpr int PG_PREFIX_OFF = 256;               // FWD / DGRAD: tiles before every expert, int [513]
 
 // Shared memory: barriers, the tile prefix, {first row, rows} of every expert (every role looks one up per tile, and the
@@ -46,13 +45,24 @@ struct PairSmem {
   static constexpr int SEG_OFF = WGRAD ? 256 : 2312;
   static constexpr int SEG_MAX = WGRAD ? 352 : 512;        // experts with an entry; the others' are read from memory
   static constexpr int CTRL = WGRAD ? 3072 : 7168;
-  static constexpr int STORE_OFF = CTRL + PG_STAGES * PG_STAGE;
+  static constexpr int RING = WGRAD ? 5 * 2 * PG_OPERAND : 172 * 1024;     // what the rest leaves of the SM's 227 KB
+  static constexpr int STORE_OFF = CTRL + RING;
   static constexpr int STORE_BUF = WGRAD ? 16384 : 8192;   // 128 rows x 64 columns, or 32 rows x 128 columns
   static constexpr int STORE_BUFS = WGRAD ? 2 : 3;         // per epilogue group
   static constexpr int STORE = STORE_BUF * STORE_BUFS;
   static constexpr int TOTAL = STORE_OFF + 2 * STORE;
   static_assert(SEG_OFF + SEG_MAX * 8 <= CTRL && CTRL % 1024 == 0 && TOTAL <= 232448, "shared memory budget");
 };
+
+// A stage holds 128 rows of the M operand and, for every chunk of rows up to `units` long, half of it in boxes of 32 rows.
+// Short chunks leave room for more stages: 8 of 20 KB up to 64 rows, 7 up to 128, 6 up to 192, 5 of 32 KB.  With few rows per
+// expert the product is bound by streaming the weights, and so by what is in flight: 32 experts x 37 rows, 2880 -> 2880, 104 us
+// with 5 stages for every length, 97 with these.
+__device__ __forceinline__ int pg_stage_bytes(int units) { return PG_OPERAND + (units + 1) / 2 * 4096; }
+__device__ __forceinline__ int pg_stages(int units) { return 9 - (units + 1) / 2; }
+static_assert(PG_MAX_STAGES * (PG_OPERAND + 4096) <= 172 * 1024 && 7 * (PG_OPERAND + 8192) <= 172 * 1024 &&
+              6 * (PG_OPERAND + 12288) <= 172 * 1024 && 5 * 2 * PG_OPERAND <= 172 * 1024, "ring");
+
 constexpr int PG_UNIT = 32;                      // rows per unit of an expert's chunk (the MMA's step in n)
 constexpr int PG_MAX_UNITS = 8;
 constexpr int PG_TILE_UNITS = 3;                 // what a tile costs beside its rows, in units (see pg_plan_tiles)
@@ -230,8 +240,8 @@ __device__ __forceinline__ void pg_uniform(PairTile& ti) {
 // whatever n is.  Over 78 products (13 dense and 11 grouped shapes, 128 to 20000 rows, forward and input gradient) the choice is
 // within 0.3 % of the best of all eight in the mean and 5 % at worst; with n + 32 it was 2.1 % and 26 % (input gradient of
 // [4096, 7168] x [2048, 7168] 108.8 us in chunks of 160 where 256 take 90.3).
-// One warp; writes the segments and the tile prefix over experts and returns the choice.
-__device__ __forceinline__ int pg_plan_tiles(const PairParams& p, int obs, int pairs, int* prefix, int2* segs) {
+// One warp; writes the segments and the tile prefix over experts, and returns the choice and a bound on the chunks it makes.
+__device__ __forceinline__ int2 pg_plan_tiles(const PairParams& p, int obs, int pairs, int* prefix, int2* segs) {
   const int lane = threadIdx.x & 31;
   int units[16], total = 0;
 #pragma unroll
@@ -259,11 +269,12 @@ __device__ __forceinline__ int pg_plan_tiles(const PairParams& p, int obs, int p
     if (cost < best_cost) { best_cost = cost; best = mu; }
   }
   best = warp_uniform(best);
-  int acc = 0;
+  int acc = 0, longest = 1;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     if (i * 32 >= p.E) break;
     const int tiles = (units[i] + best - 1) / best * obs;
+    longest = max(longest, min(units[i], best));
     int inc = tiles;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -275,7 +286,7 @@ __device__ __forceinline__ int pg_plan_tiles(const PairParams& p, int obs, int p
     acc += __shfl_sync(0xffffffffu, inc, 31);
   }
   if (lane == 0) prefix[p.E] = acc;
-  return best;
+  return make_int2(best, __reduce_max_sync(0xffffffffu, longest));
 }
 
 // Tensor maps.  w: M-side operand (weights; WGRAD: dY), x: N-side operand in boxes of 32, 64, 96 and 128 rows (WGRAD: x[2]
@@ -292,13 +303,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   constexpr int BKE = FP8 ? 128 : 64;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);           // first CTA's copy counts both CTAs' bytes
-  uint64_t* empty_bar = full_bar + PG_STAGES;
-  uint64_t* tfull_bar = empty_bar + PG_STAGES;
+  uint64_t* empty_bar = full_bar + PG_MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + PG_MAX_STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;                             // first CTA's copy counts both CTAs' epilogue warps
   uint64_t* old_bar = tempty_bar + 2;                               // WGRAD, accumulate: a chunk of the old result is here (two per group)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(old_bar + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* units_slot = reinterpret_cast<int*>(tmem_slot + 2);
+  int2* units_slot = reinterpret_cast<int2*>(tmem_slot + 2);        // largest chunk allowed, and none is longer than
   int* prefix = reinterpret_cast<int*>(smem + PG_PREFIX_OFF);
   int2* segs = reinterpret_cast<int2*>(smem + L::SEG_OFF);
   uint8_t* ring = smem + L::CTRL;
@@ -310,7 +321,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
 
   if (threadIdx.x == 0) {
     if (smem_u32(smem) & 1023u) atomicCAS(p.status, 0, ST_BAD_INDEX);   // the runtime aligns it; swizzled tiles rely on it
-    for (int s = 0; s < PG_STAGES; ++s) {
+    for (int s = 0; s < PG_MAX_STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -331,7 +342,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   if (MODE != PG_WGRAD && warp == 2) {
-    const int mu = pg_plan_tiles(p, (out_cols + 255) >> 8, pairs, prefix, segs);
+    const int2 mu = pg_plan_tiles(p, (out_cols + 255) >> 8, pairs, prefix, segs);
     if (lane == 0) *units_slot = mu;
   }
   if (MODE == PG_WGRAD)
@@ -342,8 +353,18 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   pg_cluster_sync();                              // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int max_units = MODE == PG_WGRAD ? 0 : *units_slot;
+  const int max_units = MODE == PG_WGRAD ? 0 : units_slot->x;
   const int tiles = warp_uniform(MODE == PG_WGRAD ? ((p.N + 255) >> 8) * ((p.K + p.width - 1) / p.width) * p.E : prefix[p.E]);
+  const int stage_bytes = MODE == PG_WGRAD ? 2 * PG_OPERAND : warp_uniform(pg_stage_bytes(units_slot->y));
+  // A pair with fewer tiles than others takes its share of the ring only: with few rows the launch is bound by memory, and the
+  // pairs that have most to fetch should have most in flight (8 experts x 25 rows, 224 tiles of 4096 x 256: 87 -> 80 us; 96
+  // tiles of 5760 x 256: 65 -> 55).
+  const float waves = __fdividef((float)tiles, (float)pairs);
+  int stages = MODE == PG_WGRAD ? 5 : pg_stages(units_slot->y);
+  const int each = (int)waves;                    // (both CTAs and all roles get the same, whatever it is rounded to)
+  if (pair >= tiles - each * pairs && tiles > each * pairs)
+    stages = max((int)ceilf(__fdividef((float)(stages * each), (float)(each + 1))), 2);
+  stages = warp_uniform(stages);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -381,7 +402,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       for (int ks = 0; ks < ti.ksteps; ++ks) {
         ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
         if (!ok) break;
-        const uint32_t w_dst = ring_addr + s * PG_STAGE, x_dst = w_dst + PG_OPERAND, bar = bar0 + s * 8;
+        const uint32_t w_dst = ring_addr + s * stage_bytes, x_dst = w_dst + PG_OPERAND, bar = bar0 + s * 8;
         if (elect_one()) {
           if (cta == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
           if (W_MN) pg_load_panels(w_dst, &maps.w, bar, (MODE == PG_WGRAD ? ti.row0 : w_row) + ks * BKE, m0 >> 6);
@@ -389,13 +410,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           if (X_MN) pg_load_panels(x_dst, x_map, bar, ti.row0 + ks * BKE, x0 >> 6);
           else pg_load_2d(x_dst, x_map, bar, ks * BKE, x0);
         }
-        if (++s == PG_STAGES) { s = 0; ph ^= 1; }
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
     }
     // the first CTA's commits arrive on both CTAs: all of them have before this CTA may leave
-    for (int i = 0; ok && i < PG_STAGES; ++i) {
+    for (int i = 0; ok && i < stages; ++i) {
       ok = mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
-      if (++s == PG_STAGES) { s = 0; ph ^= 1; }
+      if (++s == stages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (first CTA, for both)
@@ -427,7 +448,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           ok = mbar_wait_warp(&full_bar[s], ph, abort_flag, p.status, ST_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t wd = wd0 + (uint32_t)(s * (PG_STAGE >> 4)), xd = xd0 + (uint32_t)(s * (PG_STAGE >> 4));
+          const uint64_t wd = wd0 + (uint32_t)(s * (stage_bytes >> 4)), xd = xd0 + (uint32_t)(s * (stage_bytes >> 4));
           if (elect_one()) {
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4)
@@ -437,7 +458,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
             if (ks == ti.ksteps - 1) pg_commit_both(&tfull_bar[buf]);
           }
           left -= 4;
-          if (++s == PG_STAGES) { s = 0; ph ^= 1; }
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
         ++it;
       }

@@ -33,27 +33,34 @@ SIZES = [([1], 64, 64), ([31, 32, 33], 64, 192), ([255, 256, 257], 192, 128), ([
          ([1100, 3], 128, 320), ([700] * 9, 576, 448), ([2] * 400, 64, 128)]
 
 
+# CTAs a launch may take: all of them (a tile per pair at these sizes), and so few that a pair walks many tiles, which carries the
+# ring's and the accumulators' phases, staging buffers and old results over from tile to tile (odd values round down to pairs)
+CTAS = [0, 1, 2, 3, 7]
+
+
+@pytest.mark.parametrize("ctas", CTAS)
 @pytest.mark.parametrize("counts,n,k", SIZES)
-def test_rows_against_64_bits(counts, n, k):
+def test_rows_against_64_bits(counts, n, k, ctas):
     from system_lab_b200.ops import cuda
     a, dy, w, off, cnt = _operands(counts, n, k, 1)
     for mode, x, cols in ((0, a, n), (1, dy, k)):
         out = torch.full((x.shape[0], cols), float("nan"), device="cuda", dtype=torch.bfloat16)
-        cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k, out=out)
+        cuda.grouped_gemm_raw(mode, x, w, off, cnt, n, k, out=out, max_ctas=ctas)
         for e, (o, c) in enumerate(zip(off.tolist(), counts)):
             we = w[e].double().t() if mode == 0 else w[e].double()
             _close(out[o:o + c], x[o:o + c].double() @ we, x[o:o + c].double().abs() @ we.abs())
             assert not bool(out[o + c:o + (c + 127) // 128 * 128].any())     # padding rows are zero
 
 
+@pytest.mark.parametrize("ctas", CTAS)
 @pytest.mark.parametrize("counts,n,k", SIZES)
-def test_weight_gradient_against_64_bits(counts, n, k):
+def test_weight_gradient_against_64_bits(counts, n, k, ctas):
     from system_lab_b200.ops import cuda
     a, dy, w, off, cnt = _operands(counts, n, k, 2)
     out = torch.full_like(w, float("nan"))
-    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=out)
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=out, max_ctas=ctas)
     twice = w.clone()
-    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=twice, accumulate=True)
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=twice, accumulate=True, max_ctas=ctas)
     for e, (o, c) in enumerate(zip(off.tolist(), counts)):
         d, x = dy[o:o + c].double(), a[o:o + c].double()
         _close(out[e], d.t() @ x, d.abs().t() @ x.abs())
@@ -75,13 +82,14 @@ def test_one_segment_that_ends_inside_a_tile(rows):
     _close(dw, guard[:rows].double().t() @ x.double(), guard[:rows].double().abs().t() @ x.double().abs())
 
 
+@pytest.mark.parametrize("ctas", CTAS)
 @pytest.mark.parametrize("counts,n,k", [([1], 64, 128), ([31, 0, 257], 192, 256), ([700, 130], 320, 768)])
-def test_row_scaled_e4m3(counts, n, k):
+def test_row_scaled_e4m3(counts, n, k, ctas):
     from system_lab_b200.ops import cuda
     a, _, w, off, cnt = _operands(counts, n, k, 4)
     aq, sa = cuda.quant_rowwise(a)
     wq, sw = cuda.quant_rowwise(w)
-    out = cuda.grouped_gemm_fp8_rowwise_raw(aq, sa, wq, sw.contiguous(), off, cnt)
+    out = cuda.grouped_gemm_fp8_rowwise_raw(aq, sa, wq, sw.contiguous(), off, cnt, max_ctas=ctas)
     for e, (o, c) in enumerate(zip(off.tolist(), counts)):
         x = aq[o:o + c].double() * sa[o:o + c, None].double()
         m = (wq[e].double() * sw[e][:, None].double()).t()
