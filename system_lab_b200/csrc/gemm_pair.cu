@@ -178,11 +178,13 @@ struct PairTile {
   int ksteps, mmas;         // stages, and MMAs over all of them
 };
 
-// {first row, rows} of an expert's segment
+// {first row, rows} of an expert's segment: a corrupt plan must not turn into a runaway tile walk
+__device__ __forceinline__ int2 pg_clip(const PairParams& p, int2 s) {
+  if (s.x < 0 || s.x >= p.R || s.y <= 0) return make_int2(0, 0);
+  return make_int2(s.x, s.y < p.R - s.x ? s.y : p.R - s.x);
+}
 __device__ __forceinline__ int2 pg_segment(const PairParams& p, int e) {
-  const int off = p.seg_offsets[e], cnt = p.seg_counts[e];
-  if (off < 0 || off >= p.R || cnt <= 0) return make_int2(0, 0);      // a corrupt plan must not turn into a runaway tile walk
-  return make_int2(off, cnt < p.R - off ? cnt : p.R - off);
+  return pg_clip(p, make_int2(p.seg_offsets[e], p.seg_counts[e]));
 }
 
 // On entry ti.e holds the expert of the tile visited before (0 at first).
@@ -241,52 +243,55 @@ __device__ __forceinline__ void pg_uniform(PairTile& ti) {
 // within 0.3 % of the best of all eight in the mean and 5 % at worst; with n + 32 it was 2.1 % and 26 % (input gradient of
 // [4096, 7168] x [2048, 7168] 108.8 us in chunks of 160 where 256 take 90.3).
 // One warp; writes the segments and the tile prefix over experts, and returns the choice and a bound on the chunks it makes.
-__device__ __forceinline__ int2 pg_plan_tiles(const PairParams& p, int obs, int pairs, int* prefix, int2* segs) {
+__device__ __forceinline__ int2 pg_plan_tiles(const PairParams& p, int obs, int pairs, int* prefix, const int2* segs) {
   const int lane = threadIdx.x & 31;
-  int units[16], total = 0;
+  int tiles[PG_MAX_UNITS - 1], total = 0, longest = 0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int e = i * 32 + lane;
-    units[i] = 0;
-    if (e < p.E) {
-      segs[e] = pg_segment(p, e);
-      units[i] = (segs[e].y + PG_UNIT - 1) / PG_UNIT;
-    }
-    total += units[i];
+  for (int j = 0; j < PG_MAX_UNITS - 1; ++j) tiles[j] = 0;
+  // Small loops: a launch finds its instructions in no cache, and unrolled for 512 experts this took 3000 cycles of 4500 before the
+  // first copy (a launch without rows: 4.3 us for 1 expert, 5.0 for 128; 2.6 and 3.3 now).  A lane has neighbouring experts,
+  // so that one scan over the warp gives the prefix.
+  const int per = (p.E + 31) >> 5, e0 = lane * per, e1 = min(p.E, e0 + per);
+#pragma unroll 1
+  for (int e = e0; e < e1; ++e) {
+    const int u = (segs[e].y + PG_UNIT - 1) / PG_UNIT;
+    total += u;
+    longest = max(longest, u);
+#pragma unroll
+    for (int j = 0; j < PG_MAX_UNITS - 1; ++j) tiles[j] += (u + j + 1) / (j + 2);
   }
   total = __reduce_add_sync(0xffffffffu, total);
+  longest = __reduce_max_sync(0xffffffffu, longest);
   int best = PG_MAX_UNITS;
   float best_cost = INFINITY;
 #pragma unroll
   for (int mu = PG_MAX_UNITS; mu >= 2; --mu) {
-    int tiles = 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) tiles += (units[i] + mu - 1) / mu;
-    tiles = __reduce_add_sync(0xffffffffu, tiles);
+    const int t = __reduce_add_sync(0xffffffffu, tiles[mu - 2]);
     // (single precision throughout: 64-bit divisions here cost a microsecond per launch)
-    const float waves = ceilf((float)tiles * (float)obs / (float)pairs);
-    const float cost = waves * (float)(total + PG_TILE_UNITS * tiles) / (float)max(tiles, 1);
+    const float waves = ceilf(__fdividef((float)t * (float)obs, (float)pairs));
+    const float cost = __fdividef(waves * (float)(total + PG_TILE_UNITS * t), (float)max(t, 1));
     if (cost < best_cost) { best_cost = cost; best = mu; }
   }
-  best = warp_uniform(best);
-  int acc = 0, longest = 1;
+  // ceil(units / best) without a division: exact below 2^29
+  const uint32_t inverse = 0xffffffffu / (uint32_t)best + 1;
+  auto tiles_of = [&](int e) { return (int)__umulhi((segs[e].y + PG_UNIT - 1) / PG_UNIT + best - 1, inverse) * obs; };
+  int mine = 0;
+#pragma unroll 1
+  for (int e = e0; e < e1; ++e) mine += tiles_of(e);
+  int acc = mine;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    if (i * 32 >= p.E) break;
-    const int tiles = (units[i] + best - 1) / best * obs;
-    longest = max(longest, min(units[i], best));
-    int inc = tiles;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
-    }
-    const int e = i * 32 + lane;
-    if (e < p.E) prefix[e] = acc + inc - tiles;
-    acc += __shfl_sync(0xffffffffu, inc, 31);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, acc, o);
+    if (lane >= o) acc += v;
   }
-  if (lane == 0) prefix[p.E] = acc;
-  return make_int2(best, __reduce_max_sync(0xffffffffu, longest));
+  if (lane == 31) prefix[p.E] = acc;
+  acc -= mine;
+#pragma unroll 1
+  for (int e = e0; e < e1; ++e) {
+    prefix[e] = acc;
+    acc += tiles_of(e);
+  }
+  return make_int2(best, max(min(longest, best), 1));
 }
 
 // Tensor maps.  w: M-side operand (weights; WGRAD: dY), x: N-side operand in boxes of 32, 64, 96 and 128 rows (WGRAD: x[2]
@@ -302,6 +307,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   constexpr bool W_MN = MODE != PG_FWD, X_MN = MODE == PG_WGRAD;
   constexpr int BKE = FP8 ? 128 : 64;
   extern __shared__ __align__(1024) uint8_t smem[];
+  // (24 barriers side by side, see the initialisation)
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);           // first CTA's copy counts both CTAs' bytes
   uint64_t* empty_bar = full_bar + PG_MAX_STAGES;
   uint64_t* tfull_bar = empty_bar + PG_MAX_STAGES;
@@ -319,38 +325,34 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int out_cols = MODE == PG_FWD ? p.N : p.K;
 
-  if (threadIdx.x == 0) {
-    if (smem_u32(smem) & 1023u) atomicCAS(p.status, 0, ST_BAD_INDEX);   // the runtime aligns it; swizzled tiles rely on it
-    for (int s = 0; s < PG_MAX_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  if (warp == 0) {
+    if (lane < 2 * PG_MAX_STAGES + 8) {
+      mbar_init(&full_bar[lane], &full_bar[lane] == &tempty_bar[0] || &full_bar[lane] == &tempty_bar[1] ? 16 : 1);
+      fence_mbar_init();
     }
-    for (int b = 0; b < 4; ++b) mbar_init(&old_bar[b], 1);
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 16);
+    if (lane == 0) {
+      if (smem_u32(smem) & 1023u) atomicCAS(p.status, 0, ST_BAD_INDEX);   // the runtime aligns it; swizzled tiles rely on it
+      *abort_flag = 0;
+      prefetch_tmap(&maps.w);
+      prefetch_tmap(&maps.x[3]);
+      prefetch_tmap(&maps.c);
     }
-    *abort_flag = 0;
-    fence_mbar_init();
-    prefetch_tmap(&maps.w);
-    prefetch_tmap(&maps.x[3]);
-    prefetch_tmap(&maps.c);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  if (warp >= 2)
+    for (int e = threadIdx.x - 64; e < p.E && e < L::SEG_MAX; e += PG_THREADS - 64) segs[e] = pg_segment(p, e);
+  if (MODE != PG_WGRAD && warp >= 2) asm volatile("bar.sync 3, 256;" ::: "memory");
   if (MODE != PG_WGRAD && warp == 2) {
     const int2 mu = pg_plan_tiles(p, (out_cols + 255) >> 8, pairs, prefix, segs);
     if (lane == 0) *units_slot = mu;
   }
-  if (MODE == PG_WGRAD)
-    for (int e = threadIdx.x; e < p.E && e < L::SEG_MAX; e += PG_THREADS) segs[e] = pg_segment(p, e);
   tc_fence_before();
-  __syncthreads();
   __syncwarp();
-  pg_cluster_sync();                              // the peer's barriers exist before anything arrives on them
+  pg_cluster_sync();                              // this CTA's set-up is done, and the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int max_units = MODE == PG_WGRAD ? 0 : units_slot->x;
@@ -414,7 +416,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       }
     }
     // the first CTA's commits arrive on both CTAs: all of them have before this CTA may leave
-    for (int i = 0; ok && i < stages; ++i) {
+    for (int i = 0; ok && pair < tiles && i < stages; ++i) {
       ok = mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
       if (++s == stages) { s = 0; ph ^= 1; }
     }
