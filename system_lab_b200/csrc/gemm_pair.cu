@@ -69,13 +69,19 @@ constexpr int PG_TILE_UNITS = 3;                 // what a tile costs beside its
 
 enum { PG_FWD = 0, PG_DGRAD = 1, PG_WGRAD = 2 };
 
+// WGRAD: a group of epilogue warps stores a 16 KB chunk every PG_STORE_NS at most (one may come early), a little less than all of
+// them together get from memory (5.9 TB/s).  With short reductions the launch is bound by writing its result.  The groups can
+// produce it at twice that rate, and memory serves the SMs unevenly: those it favours end at 67 us of 92 and the others go on
+// alone (8 experts x 25 rows into [4096, 7168], 470 MB).  Paced, all end together: 98 -> 86 us; 32 experts x 37 rows 410 -> 325,
+// into [5760, 2880] 236 -> 198.  780 ns gives 84 there but 396 and 242, 840 ns with four chunks early 88, 332 and 234.
+constexpr uint64_t PG_STORE_NS = 820;
+
 struct PairParams {
   const int* seg_offsets;
   const int* seg_counts;
   int E, R, N, K;
   int width;                // WGRAD: columns of a tile, 256 or 128
   __nv_bfloat16* C;
-  int accumulate;           // WGRAD only
   const float* sa;          // e4m3: [R]
   const float* sb;          // e4m3: [E, N]
   int* status;
@@ -300,7 +306,8 @@ struct PairMaps {
   CUtensorMap w, c, x[4];
 };
 
-template <int MODE, bool FP8>
+// ACC: WGRAD adds to the old result.
+template <int MODE, bool FP8, bool ACC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   using L = PairSmem<MODE>;
@@ -474,6 +481,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
     uint64_t* const old_g = old_bar + 2 * grp;
     int it = 0, ctr = 0;
     int slot = 0;                                 // FWD / DGRAD: staging buffer in turn
+    uint64_t due = 0;                             // WGRAD: when this group's next chunk may be stored
     bool ok = true;                               // no wait of this warp has run out (see mbar_wait_warp)
     PairTile ti;
     ti.e = 0;
@@ -483,16 +491,15 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       const int m0 = ti.ob * 256 + (int)cta * 128;
       const int buf = it & 1;
       const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * 256;
-      // Rows of the output block beyond the expert's N: the 2-D output map cannot clip at an expert boundary, so such a block
-      // goes through guarded global accesses.  All others leave by TMA, and a sum onto the old result has that brought in
-      // by TMA as well (a thread's own row is a line per access when read from global memory), one chunk ahead.
-      const bool hangs = MODE == PG_WGRAD && m0 + 128 > p.N;
-      if (MODE == PG_WGRAD && p.accumulate && !empty && !hangs && ok && store_thread) {
-        if (ti.cb * ti.width + grp * 64 < p.K && grp * 64 < ti.width) {
-          tma_store_wait_read<0>();
-          mbar_arrive_expect_tx(&old_g[ctr & 1], 16384);
-          tma_load_2d(stage + (ctr & 1) * 16384, &maps.c, &old_g[ctr & 1], ti.cb * ti.width + grp * 64, ti.e * p.N + m0);
-        }
+      // WGRAD: 64-column chunks of this CTA's 128 rows (none beyond the expert's N; the output map clips a block that hangs over
+      // it).  A sum onto the old result has that brought in by TMA too (a thread's own row is a line per access when read from
+      // global memory), one chunk ahead.
+      const int col0 = ti.cb * ti.width;
+      const int chunks = m0 >= p.N || (ACC && empty) ? 0 : min(ti.width, p.K - col0) >> 6;
+      if (ACC && grp < chunks && ok && store_thread) {
+        tma_store_wait_read<0>();
+        mbar_arrive_expect_tx(&old_g[ctr & 1], 16384);
+        tma_load_3d(stage + (ctr & 1) * 16384, &maps.c, &old_g[ctr & 1], col0 + grp * 64, m0, ti.e);
       }
       // e4m3: channel scales (channels lane / 4 + 0, 8, 16, 24 of this warp's 32) and the scale of row `lane` of the group's
       // first step are requested before the accumulator is waited for
@@ -582,10 +589,6 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         }
       } else {
         const int r_in_tile = lg * 32 + lane;
-        const int col0 = ti.cb * ti.width;
-        const bool row_ok = m0 + r_in_tile < p.N;
-        __nv_bfloat16* c_row = p.C + ((size_t)ti.e * p.N + m0 + r_in_tile) * p.K;
-        const int chunks = (empty && p.accumulate) ? 0 : min(ti.width, p.K - col0) >> 6;
 #pragma unroll 1
         for (int c = grp; c < chunks; c += 2) {
           uint32_t lo[32], hi[32];
@@ -597,33 +600,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) lo[i] = hi[i] = 0u;
           }
-          if (hangs) {
-            if (ok && row_ok) {
-#pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                const uint32_t* v = g < 4 ? lo + g * 8 : hi + (g - 4) * 8;
-                float f[8], o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[i]);
-                bf16x8* dst = reinterpret_cast<bf16x8*>(c_row + col0 + c * 64 + g * 8);
-                if (p.accumulate) {
-                  unpack8(*dst, o);
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) f[i] += o[i];
-                }
-                *dst = pack8(f);
-              }
-            }
-            continue;
-          }
           uint8_t* sbuf = stage + (ctr & 1) * 16384;
-          if (p.accumulate) {
+          if (ACC) {
             ok = ok && mbar_wait_warp(&old_g[ctr & 1], (ctr >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
             if (ok && store_thread && c + 2 < chunks) {   // the group's next chunk, into the buffer whose store came before this one
               tma_store_wait_read<0>();
               mbar_arrive_expect_tx(&old_g[(ctr + 1) & 1], 16384);
-              tma_load_2d(stage + ((ctr + 1) & 1) * 16384, &maps.c, &old_g[(ctr + 1) & 1], col0 + c * 64 + 128,
-                          ti.e * p.N + m0);
+              tma_load_3d(stage + ((ctr + 1) & 1) * 16384, &maps.c, &old_g[(ctr + 1) & 1], col0 + c * 64 + 128, m0, ti.e);
             }
           } else {
             if (store_thread) tma_store_wait_read<1>();
@@ -636,7 +619,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
             float f[8], o[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[i]);
-            if (p.accumulate) {
+            if (ACC) {
               unpack8(*dst, o);
 #pragma unroll
               for (int i = 0; i < 8; ++i) f[i] += o[i];
@@ -645,8 +628,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           }
           fence_proxy_async();
           pg_group_sync(grp);
+          if (store_thread) {                     // see PG_STORE_NS
+            uint64_t now = globaltimer_ns();
+            for (int spins = 0; now < due && spins < 1000; ++spins) now = globaltimer_ns();
+            due = max(due + PG_STORE_NS, now);
+          }
           if (ok && store_thread) {
-            tma_store_2d(&maps.c, sbuf, col0 + c * 64, ti.e * p.N + m0);
+            tma_store_3d(&maps.c, sbuf, col0 + c * 64, m0, ti.e);
             tma_store_commit();
           }
           ++ctr;
@@ -679,7 +667,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   }
 }
 
-template <int MODE, bool FP8>
+template <int MODE, bool FP8, bool ACC = false>
 static int pg_launch(const void* A, const void* B, const PairParams& p, int max_ctas, cudaStream_t stream) {
   constexpr CUtensorMapDataType DT = FP8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   constexpr int ES = FP8 ? 1 : 2, BKE = FP8 ? 128 : 64;
@@ -691,7 +679,7 @@ static int pg_launch(const void* A, const void* B, const PairParams& p, int max_
     if ((rc = tma_make_map_2d(&m.x[3], B, DT, ES, p.R, p.K, p.K, 64, 64, 2))) return rc;
     if ((rc = tma_make_map_2d(&m.x[2], B, DT, ES, p.R, p.K, p.K, 64, 64, 1))) return rc;
     m.x[0] = m.x[1] = m.x[2];
-    if ((rc = tma_make_map_bf16(&m.c, p.C, wrows, p.K, 128, 64))) return rc;
+    if ((rc = tma_make_map_2d(&m.c, p.C, DT, ES, p.N, p.K, p.K, 128, 64, -p.E))) return rc;
   } else {
     const int red = MODE == PG_FWD ? p.K : p.N;
     if (MODE == PG_FWD) rc = tma_make_map_2d(&m.w, B, DT, ES, wrows, p.K, p.K, 128, BKE);
@@ -701,7 +689,7 @@ static int pg_launch(const void* A, const void* B, const PairParams& p, int max_
       if ((rc = tma_make_map_2d(&m.x[i], A, DT, ES, p.R, red, red, 32 * (i + 1), BKE))) return rc;
     if ((rc = tma_make_map_bf16(&m.c, p.C, p.R, MODE == PG_FWD ? p.N : p.K, 32, 64))) return rc;
   }
-  auto kern = pair_gemm_kernel<MODE, FP8>;
+  auto kern = pair_gemm_kernel<MODE, FP8, ACC>;
   static bool attr_set = false;
   if (!attr_set) {
     SLAB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<MODE>::TOTAL));
@@ -738,12 +726,13 @@ extern "C" int slab_grouped_gemm_bf16(int mode, const void* A, const void* B, vo
   const long pairs = (max_ctas > 1 && max_ctas < sm_count() ? max_ctas : sm_count()) / 2, obs = (long)E * ((N + 255) / 256);
   const long waves256 = (obs * ((K + 255) / 256) + pairs - 1) / pairs, waves128 = (obs * ((K + 127) / 128) + pairs - 1) / pairs;
   const int width = waves128 * 62 < waves256 * 100 ? 128 : 256;
-  PairParams p{seg_offsets, seg_counts, E, R, N, K, width, static_cast<__nv_bfloat16*>(C), accumulate, nullptr, nullptr, status,
-               ready, ready_world, ready_epoch, slab_moe_wait_limit_ns()};
+  PairParams p{seg_offsets, seg_counts, E, R, N, K, width, static_cast<__nv_bfloat16*>(C), nullptr, nullptr, status, ready, ready_world, ready_epoch, slab_moe_wait_limit_ns()};
   switch (mode) {
     case PG_FWD: return pg_launch<PG_FWD, false>(A, B, p, max_ctas, stream);
     case PG_DGRAD: return pg_launch<PG_DGRAD, false>(A, B, p, max_ctas, stream);
-    case PG_WGRAD: return pg_launch<PG_WGRAD, false>(A, B, p, max_ctas, stream);
+    case PG_WGRAD:
+      return accumulate ? pg_launch<PG_WGRAD, false, true>(A, B, p, max_ctas, stream)
+                        : pg_launch<PG_WGRAD, false>(A, B, p, max_ctas, stream);
   }
   return -101;
 }
@@ -754,7 +743,7 @@ extern "C" int slab_grouped_gemm_fp8_rowwise(const void* A, const float* sa, con
                                              int K, int max_ctas, int* status, cudaStream_t stream) {
   using namespace slab;
   if (E > 512 || K % 128 || N % 64) return -100;
-  PairParams p{seg_offsets, seg_counts, E, R, N, K, 256, static_cast<__nv_bfloat16*>(C), 0, sa, sb, status,
+  PairParams p{seg_offsets, seg_counts, E, R, N, K, 256, static_cast<__nv_bfloat16*>(C), sa, sb, status,
                nullptr, 0, 0, 0};
   return pg_launch<PG_FWD, true>(A, B, p, max_ctas, stream);
 }

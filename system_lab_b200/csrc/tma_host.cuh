@@ -49,7 +49,7 @@ constexpr int TMA_CACHE_SLOTS = 1024;   // direct mapped; a colliding entry is s
 inline uint64_t tma_key_hash(const TmaMapKey& k) {
   uint64_t h = 1469598103934665603ull;
   const uint64_t parts[6] = {reinterpret_cast<uint64_t>(k.base), k.rows, k.cols, k.row_stride_bytes,
-                             (uint64_t(k.box_rows) << 32) | k.box_cols, (uint64_t(k.panels) << 32) | uint64_t(k.dtype)};
+                             (uint64_t(k.box_rows) << 32) | k.box_cols, (uint64_t(uint32_t(k.panels)) << 32) | uint64_t(k.dtype)};
   for (int i = 0; i < 6; ++i) {
     h ^= parts[i];
     h *= 1099511628211ull;
@@ -65,9 +65,11 @@ inline uint64_t tma_key_hash(const TmaMapKey& k) {
 // `panels` > 0: the same tensor seen as panels of `box_cols` columns (which `cols` is a multiple of and which are one
 // 128-byte swizzle row); coordinates are (0, row, panel) and a box covers `panels` neighbouring ones, each landing as
 // [box_rows][128 bytes] behind the one before: one copy for an operand several swizzle rows wide.
+// `panels` < 0: -panels matrices [rows, cols], one behind the other; coordinates are (column, row, matrix), a box lies in one
+// matrix, and what hangs over its last row is clipped there instead of running into the next one.
 inline int tma_make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int esize, uint64_t rows,
                            uint64_t cols, uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols,
-                           uint32_t panels = 0) {
+                           int panels = 0) {
   static thread_local TmaMapSlot* cache = nullptr;
   static thread_local bool ctx_ready = false;
   TmaMapKey key;
@@ -79,7 +81,7 @@ inline int tma_make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType
   key.box_rows = box_rows;
   key.box_cols = box_cols;
   key.dtype = (int)dt;
-  key.panels = (int)panels;
+  key.panels = panels;
   if (!cache) cache = new TmaMapSlot[TMA_CACHE_SLOTS]();
   TmaMapSlot& slot = cache[tma_key_hash(key) % TMA_CACHE_SLOTS];
   if (slot.used && memcmp(&slot.key, &key, sizeof(key)) == 0) {
@@ -94,9 +96,9 @@ inline int tma_make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType
     cudaFree(0);
     ctx_ready = true;
   }
-  cuuint64_t dims[3] = {panels ? box_cols : cols, rows, panels ? cols / box_cols : 1};
-  cuuint64_t strides[2] = {key.row_stride_bytes, (cuuint64_t)box_cols * esize};
-  cuuint32_t box[3] = {box_cols, box_rows, panels ? panels : 1};
+  cuuint64_t dims[3] = {panels > 0 ? box_cols : cols, rows, panels > 0 ? cols / box_cols : (cuuint64_t)-panels};
+  cuuint64_t strides[2] = {key.row_stride_bytes, panels > 0 ? (cuuint64_t)box_cols * esize : rows * key.row_stride_bytes};
+  cuuint32_t box[3] = {box_cols, box_rows, panels > 0 ? (cuuint32_t)panels : 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(m, dt, panels ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

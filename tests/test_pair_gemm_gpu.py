@@ -30,7 +30,8 @@ def _close(out, ref, magnitude):
 
 # rows around the 32-row unit, the 256-row chunk and uneven cuts; output columns around the 64-, 128- and 256-wide blocks
 SIZES = [([1], 64, 64), ([31, 32, 33], 64, 192), ([255, 256, 257], 192, 128), ([0, 513, 0, 5], 320, 64),
-         ([1100, 3], 128, 320), ([700] * 9, 576, 448), ([2] * 400, 64, 128)]
+         ([1100, 3], 128, 320), ([700] * 9, 576, 448), ([2] * 400, 64, 128),
+         ([60, 0, 300, 90] * 6, 384, 320), ([1, 0, 33, 2] * 128, 64, 64)]
 
 
 # CTAs a launch may take: all of them (a tile per pair at these sizes), and so few that a pair walks many tiles, which carries the
