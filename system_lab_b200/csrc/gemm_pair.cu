@@ -5,6 +5,7 @@
 //   DGRAD  C[r, k]    = sum_n A[r, n] * B[e, n, k]     A: dY   [R, N]   B: weights [E, N, K] (MN-major operand)
 //   WGRAD  C[e, n, k] = sum_r A[r, n] * B[r, k]        A: dY   [R, N]   B: acts    [R, K]    (both MN-major)
 //   row-scaled e4m3 (FWD only): the same product times sa[r] * sb[e, n]
+//   WGRAD_T  WGRAD with the operands' sides exchanged (the tile is computed transposed), for N just over a multiple of 256
 //
 // Bound by the tensor pipe, its operand feed and, on long runs, the power cap.  What follows from that:
 //  * Two CTAs share one instruction (256 x n): each stages 128 rows of the M operand and half of the N operand, so a CTA
@@ -67,7 +68,8 @@ constexpr int PG_UNIT = 32;                      // rows per unit of an expert's
 constexpr int PG_MAX_UNITS = 8;
 constexpr int PG_TILE_UNITS = 3;                 // what a tile costs beside its rows, in units (see pg_plan_tiles)
 
-enum { PG_FWD = 0, PG_DGRAD = 1, PG_WGRAD = 2 };
+enum { PG_FWD = 0, PG_DGRAD = 1, PG_WGRAD = 2, PG_WGRAD_T = 3 };
+__host__ __device__ constexpr bool pg_over_rows(int mode) { return mode >= PG_WGRAD; }      // the reduction runs over an expert's rows
 
 // WGRAD: a group of epilogue warps stores a 16 KB chunk every PG_STORE_NS at most (one may come early), a little less than all of
 // them together get from memory (5.9 TB/s).  With short reductions the launch is bound by writing its result.  The groups can
@@ -80,7 +82,7 @@ struct PairParams {
   const int* seg_offsets;
   const int* seg_counts;
   int E, R, N, K;
-  int width;                // WGRAD: columns of a tile, 256 or 128
+  int width;                // WGRAD: columns of a tile on the N side, 256 or 128
   __nv_bfloat16* C;
   const float* sa;          // e4m3: [R]
   const float* sb;          // e4m3: [E, N]
@@ -198,8 +200,9 @@ template <int MODE, bool FP8>
 __device__ __forceinline__ void pg_get_tile(int t, const int* prefix, const int2* segs, int max_units, const PairParams& p,
                                             PairTile& ti) {
   constexpr int BKE = FP8 ? 128 : 64;
-  if (MODE == PG_WGRAD) {
-    const int obs = (p.N + 255) >> 8, per = obs * ((p.K + p.width - 1) / p.width);
+  if (pg_over_rows(MODE)) {
+    const int side_m = MODE == PG_WGRAD_T ? p.K : p.N, side_n = MODE == PG_WGRAD_T ? p.N : p.K;
+    const int obs = (side_m + 255) >> 8, per = obs * ((side_n + p.width - 1) / p.width);
     ti.e = t / per;
     ti.zero_steps = 0;
     const int local = t - ti.e * per;
@@ -209,7 +212,7 @@ __device__ __forceinline__ void pg_get_tile(int t, const int* prefix, const int2
     const int rows = seg.y;
     ti.row0 = seg.x;
     ti.width = p.width;
-    ti.n = p.K - ti.cb * p.width > 128 ? p.width : 128;          // half of it is whole 64-column panels; what lies beyond K reads as zero
+    ti.n = side_n - ti.cb * p.width > 128 ? p.width : 128;       // half of it is whole 64-column panels; what lies beyond reads as zero
     ti.ksteps = (rows + BKE - 1) / BKE;
     ti.mmas = (rows + 15) >> 4;                          // rows behind the last valid one are zero: whole MMAs of them are left out
     return;
@@ -311,7 +314,8 @@ template <int MODE, bool FP8, bool ACC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   using L = PairSmem<MODE>;
-  constexpr bool W_MN = MODE != PG_FWD, X_MN = MODE == PG_WGRAD;
+  constexpr bool RED = pg_over_rows(MODE);
+  constexpr bool W_MN = MODE != PG_FWD, X_MN = RED;
   constexpr int BKE = FP8 ? 128 : 64;
   extern __shared__ __align__(1024) uint8_t smem[];
   // (24 barriers side by side, see the initialisation)
@@ -352,8 +356,8 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   }
   if (warp >= 2)
     for (int e = threadIdx.x - 64; e < p.E && e < L::SEG_MAX; e += PG_THREADS - 64) segs[e] = pg_segment(p, e);
-  if (MODE != PG_WGRAD && warp >= 2) asm volatile("bar.sync 3, 256;" ::: "memory");
-  if (MODE != PG_WGRAD && warp == 2) {
+  if (!RED && warp >= 2) asm volatile("bar.sync 3, 256;" ::: "memory");
+  if (!RED && warp == 2) {
     const int2 mu = pg_plan_tiles(p, (out_cols + 255) >> 8, pairs, prefix, segs);
     if (lane == 0) *units_slot = mu;
   }
@@ -362,14 +366,15 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
   pg_cluster_sync();                              // this CTA's set-up is done, and the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int max_units = MODE == PG_WGRAD ? 0 : units_slot->x;
-  const int tiles = warp_uniform(MODE == PG_WGRAD ? ((p.N + 255) >> 8) * ((p.K + p.width - 1) / p.width) * p.E : prefix[p.E]);
-  const int stage_bytes = MODE == PG_WGRAD ? 2 * PG_OPERAND : warp_uniform(pg_stage_bytes(units_slot->y));
+  const int max_units = RED ? 0 : units_slot->x;
+  const int side_m = MODE == PG_WGRAD ? p.N : p.K, side_n = MODE == PG_WGRAD ? p.K : p.N;
+  const int tiles = warp_uniform(RED ? ((side_m + 255) >> 8) * ((side_n + p.width - 1) / p.width) * p.E : prefix[p.E]);
+  const int stage_bytes = RED ? 2 * PG_OPERAND : warp_uniform(pg_stage_bytes(units_slot->y));
   // A pair with fewer tiles than others takes its share of the ring only: with few rows the launch is bound by memory, and the
   // pairs that have most to fetch should have most in flight (8 experts x 25 rows, 224 tiles of 4096 x 256: 87 -> 80 us; 96
   // tiles of 5760 x 256: 65 -> 55).
   const float waves = __fdividef((float)tiles, (float)pairs);
-  int stages = MODE == PG_WGRAD ? 5 : pg_stages(units_slot->y);
+  int stages = RED ? 5 : pg_stages(units_slot->y);
   const int each = (int)waves;                    // (both CTAs and all roles get the same, whatever it is rounded to)
   if (pair >= tiles - each * pairs && tiles > each * pairs)
     stages = max((int)ceilf(__fdividef((float)(stages * each), (float)(each + 1))), 2);
@@ -388,7 +393,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
     for (int t = pair; ok && t < tiles; t += pairs) {
       pg_get_tile<MODE, FP8>(t, prefix, segs, max_units, p, ti);
       pg_uniform(ti);
-      if (MODE != PG_WGRAD && p.ready != nullptr && ti.e != last_e) {
+      if (!RED && p.ready != nullptr && ti.e != last_e) {
         // rows arrive expert by expert from the sources: one flag per lane; the proxy fence orders the TMA reads
         // behind the acquired generic-proxy stores
         bool mine = true;
@@ -406,7 +411,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
       const int units = X_MN ? 4 : (half + 31) >> 5;
       const uint32_t bytes = 2u * (PG_OPERAND + (X_MN ? half * 128 : units * 4096));      // of both CTAs
       const int w_row = ti.e * p.N, m0 = ti.ob * 256 + (int)cta * 128;
-      const int x0 = MODE == PG_WGRAD ? ti.cb * p.width + (int)cta * half : ti.row0 + (int)cta * half;
+      const int x0 = RED ? ti.cb * p.width + (int)cta * half : ti.row0 + (int)cta * half;
       const CUtensorMap* x_map = &maps.x[X_MN ? (half == 128 ? 3 : 2) : units - 1];
       for (int ks = 0; ks < ti.ksteps; ++ks) {
         ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
@@ -414,7 +419,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         const uint32_t w_dst = ring_addr + s * stage_bytes, x_dst = w_dst + PG_OPERAND, bar = bar0 + s * 8;
         if (elect_one()) {
           if (cta == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
-          if (W_MN) pg_load_panels(w_dst, &maps.w, bar, (MODE == PG_WGRAD ? ti.row0 : w_row) + ks * BKE, m0 >> 6);
+          if (W_MN) pg_load_panels(w_dst, &maps.w, bar, (RED ? ti.row0 : w_row) + ks * BKE, m0 >> 6);
           else pg_load_2d(w_dst, &maps.w, bar, ks * BKE, w_row + m0);
           if (X_MN) pg_load_panels(x_dst, x_map, bar, ti.row0 + ks * BKE, x0 >> 6);
           else pg_load_2d(x_dst, x_map, bar, ks * BKE, x0);
@@ -461,7 +466,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           if (elect_one()) {
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4)
-              if (MODE != PG_WGRAD || k4 < left)
+              if (!RED || k4 < left)
                 pg_mma<FP8>(d, wd + k4 * W_STEP, xd + k4 * X_STEP, idesc, (ks | k4) != 0 ? 1u : 0u);
             pg_commit_both(&empty_bar[s]);
             if (ks == ti.ksteps - 1) pg_commit_both(&tfull_bar[buf]);
@@ -487,7 +492,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
     ti.e = 0;
     for (int t = pair; t < tiles; t += pairs) {
       pg_get_tile<MODE, FP8>(t, prefix, segs, max_units, p, ti);
-      const bool empty = ti.ksteps == 0;          // WGRAD of an expert without rows: its gradient is zero
+      const bool empty = RED && ti.ksteps == 0;   // an expert without rows: its weight gradient is zero
       const int m0 = ti.ob * 256 + (int)cta * 128;
       const int buf = it & 1;
       const uint32_t taddr = tmem_base + (uint32_t(lg * 32) << 16) + buf * 256;
@@ -518,12 +523,14 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
         tc_fence_after();
       }
       if (MODE != PG_WGRAD) {
-        const int steps = ti.n / PG_UNIT;
-        bool held = true;                         // this warp has not handed the accumulator back yet
+        const int first = MODE == PG_WGRAD_T ? ti.cb * ti.width : ti.row0;
+        const int all = MODE == PG_WGRAD_T ? min(ti.width, p.N - first) / PG_UNIT : ti.n / PG_UNIT + ti.zero_steps;
+        const int steps = MODE != PG_WGRAD_T ? ti.n / PG_UNIT : empty ? 0 : all;
+        bool held = !empty;                       // this warp has not handed the accumulator back yet
 #pragma unroll 1
-        for (int st = grp; st < steps + ti.zero_steps; st += 2) {
+        for (int st = grp; st < all; st += 2) {
           // rows 8j + 2 (lane % 4) and the next one of this step's 32
-          const int row = ti.row0 + st * PG_UNIT;
+          const int row = first + st * PG_UNIT;
           uint32_t v[2][16];
           float sa[4][2];
           if (st < steps) {
@@ -576,8 +583,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, const PairParams p) {
           pg_group_sync(grp);
           if (ok && store_thread) {
             const uint8_t* b = stage + slot * L::STORE_BUF;
-            if (m0 < out_cols && row < p.R) tma_store_2d(&maps.c, b, m0, row);
-            if (m0 + 64 < out_cols && row < p.R) tma_store_2d(&maps.c, b + 4096, m0 + 64, row);
+            if (MODE == PG_WGRAD_T) {
+              if (m0 < out_cols) tma_store_3d(&maps.c, b, m0, row, ti.e);
+              if (m0 + 64 < out_cols) tma_store_3d(&maps.c, b + 4096, m0 + 64, row, ti.e);
+            } else {
+              if (m0 < out_cols && row < p.R) tma_store_2d(&maps.c, b, m0, row);
+              if (m0 + 64 < out_cols && row < p.R) tma_store_2d(&maps.c, b + 4096, m0 + 64, row);
+            }
             tma_store_commit();
           }
           if (++slot == L::STORE_BUFS) slot = 0;
@@ -674,12 +686,15 @@ static int pg_launch(const void* A, const void* B, const PairParams& p, int max_
   PairMaps m;
   const uint64_t wrows = (uint64_t)p.E * p.N;
   int rc;
-  if (MODE == PG_WGRAD) {
-    if ((rc = tma_make_map_2d(&m.w, A, DT, ES, p.R, p.N, p.N, 64, 64, 2))) return rc;
-    if ((rc = tma_make_map_2d(&m.x[3], B, DT, ES, p.R, p.K, p.K, 64, 64, 2))) return rc;
-    if ((rc = tma_make_map_2d(&m.x[2], B, DT, ES, p.R, p.K, p.K, 64, 64, 1))) return rc;
+  if (pg_over_rows(MODE)) {
+    const bool t = MODE == PG_WGRAD_T;
+    const void *w = t ? B : A, *x = t ? A : B;
+    const int side_m = t ? p.K : p.N, side_n = t ? p.N : p.K;
+    if ((rc = tma_make_map_2d(&m.w, w, DT, ES, p.R, side_m, side_m, 64, 64, 2))) return rc;
+    if ((rc = tma_make_map_2d(&m.x[3], x, DT, ES, p.R, side_n, side_n, 64, 64, 2))) return rc;
+    if ((rc = tma_make_map_2d(&m.x[2], x, DT, ES, p.R, side_n, side_n, 64, 64, 1))) return rc;
     m.x[0] = m.x[1] = m.x[2];
-    if ((rc = tma_make_map_2d(&m.c, p.C, DT, ES, p.N, p.K, p.K, 128, 64, -p.E))) return rc;
+    if ((rc = tma_make_map_2d(&m.c, p.C, DT, ES, p.N, p.K, p.K, t ? 32 : 128, 64, -p.E))) return rc;
   } else {
     const int red = MODE == PG_FWD ? p.K : p.N;
     if (MODE == PG_FWD) rc = tma_make_map_2d(&m.w, B, DT, ES, wrows, p.K, p.K, 128, BKE);
@@ -702,6 +717,15 @@ static int pg_launch(const void* A, const void* B, const PairParams& p, int max_
   return (int)cudaGetLastError();
 }
 
+// What the waves of tiles cost with `side_m` on the M side: a tile of 128 columns takes 0.62 of one of 256 (249 against 398 ns per
+// 64-deep step), and so does a last tile of at most 128.
+static float pg_wgrad_cost(int E, int side_m, int side_n, int width, int pairs) {
+  const int cbs = (side_n + width - 1) / width, last = side_n - (cbs - 1) * width;
+  const long tiles = (long)E * ((side_m + 255) / 256) * cbs;
+  const float mean = ((cbs - 1) * (width == 256 ? 1.f : 0.62f) + (last > 128 ? 1.f : 0.62f)) / cbs;
+  return (float)((tiles + pairs - 1) / pairs) * mean;
+}
+
 }  // namespace slab
 
 extern "C" unsigned long long slab_moe_wait_limit_ns();
@@ -721,16 +745,20 @@ extern "C" int slab_grouped_gemm_bf16(int mode, const void* A, const void* B, vo
   using namespace slab;
   if (E > 512 || K % 64 || N % 64) return -100;
   if (ready && (ready_world < 1 || ready_world > 32 || mode == PG_WGRAD)) return -102;
-  // WGRAD: tiles of 256 columns unless half of them leave fewer idle pairs in the last wave; a tile of 128 takes 0.62 of one
-  // of 256 (249 against 398 ns per 64-deep step)
-  const long pairs = (max_ctas > 1 && max_ctas < sm_count() ? max_ctas : sm_count()) / 2, obs = (long)E * ((N + 255) / 256);
-  const long waves256 = (obs * ((K + 255) / 256) + pairs - 1) / pairs, waves128 = (obs * ((K + 127) / 128) + pairs - 1) / pairs;
-  const int width = waves128 * 62 < waves256 * 100 ? 128 : 256;
+  // WGRAD: the width of tiles, and the side of the operands, whose waves cost least.  Exchanged sides have to be a tenth better: they
+  // are where N is just over a multiple of 256 (4096 rows into [576, 7168]: 52 us as three blocks of which 0.75 are empty, 37 us
+  // exchanged, 38 on one CTA per 128 x 256).  They do not add to an old result, which would have to come in transposed.
+  const int pairs = (max_ctas > 1 && max_ctas < sm_count() ? max_ctas : sm_count()) / 2;
+  const float c256 = pg_wgrad_cost(E, N, K, 256, pairs), c128 = pg_wgrad_cost(E, N, K, 128, pairs);
+  const float t256 = pg_wgrad_cost(E, K, N, 256, pairs), t128 = pg_wgrad_cost(E, K, N, 128, pairs);
+  const bool exchange = mode == PG_WGRAD && !accumulate && fminf(t256, t128) < 0.9f * fminf(c256, c128);
+  const int width = (exchange ? t128 < t256 : c128 < c256) ? 128 : 256;
   PairParams p{seg_offsets, seg_counts, E, R, N, K, width, static_cast<__nv_bfloat16*>(C), nullptr, nullptr, status, ready, ready_world, ready_epoch, slab_moe_wait_limit_ns()};
   switch (mode) {
     case PG_FWD: return pg_launch<PG_FWD, false>(A, B, p, max_ctas, stream);
     case PG_DGRAD: return pg_launch<PG_DGRAD, false>(A, B, p, max_ctas, stream);
     case PG_WGRAD:
+      if (exchange) return pg_launch<PG_WGRAD_T, false>(A, B, p, max_ctas, stream);
       return accumulate ? pg_launch<PG_WGRAD, false, true>(A, B, p, max_ctas, stream)
                         : pg_launch<PG_WGRAD, false>(A, B, p, max_ctas, stream);
   }

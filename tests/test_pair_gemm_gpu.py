@@ -68,6 +68,21 @@ def test_weight_gradient_against_64_bits(counts, n, k, ctas):
         _close(twice[e], w[e].double() + d.t() @ x, w[e].double().abs() + d.abs().t() @ x.abs())
 
 
+# N just over a multiple of 256 against a wide K: the operands change sides (which the launch's pairs decide), in tiles of 128 and
+# of 256 columns of N, with a last one of 64, 192 and 320; K that ends inside a 128- and a 64-wide half of a block
+@pytest.mark.parametrize("ctas", [0, 2, 7])
+@pytest.mark.parametrize("counts,n,k", [([200], 576, 7168), ([1], 576, 7104), ([130, 0, 33], 576, 2368), ([513, 7], 320, 3136),
+                                        ([77] * 5, 832, 4096), ([0, 40], 320, 704)])
+def test_weight_gradient_with_exchanged_sides(counts, n, k, ctas):
+    from system_lab_b200.ops import cuda
+    a, dy, w, off, cnt = _operands(counts, n, k, 6)
+    out = torch.full_like(w, float("nan"))
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=out, max_ctas=ctas)
+    for e, (o, c) in enumerate(zip(off.tolist(), counts)):
+        d, x = dy[o:o + c].double(), a[o:o + c].double()
+        _close(out[e], d.t() @ x, d.abs().t() @ x.abs())
+
+
 @pytest.mark.parametrize("rows", [1, 33, 100, 1021])
 def test_one_segment_that_ends_inside_a_tile(rows):
     from system_lab_b200.ops import cuda
