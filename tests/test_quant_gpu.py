@@ -5,10 +5,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _same_up_to_a_step(q, s, x):
-    """Half an e4m3 step (2^-4 of the value, 2^-10 of the scale's unit near zero), doubled for the kernel's reciprocal."""
+def _rounded_to_nearest(q, s, x):
+    """Half an e4m3 step: 2^-4 of the value, 2^-10 of the scale near zero.  The kernels multiply by 448 / amax in fp32, whose error
+    (2^-20 of the value at most, reciprocal and product) can turn a near-tie only."""
     d = q.double() * s.double()
-    assert bool(((d - x.double()).abs() <= x.double().abs() * 2 ** -3 + s.double() * 2 ** -9).all())
+    assert bool(((d - x.double()).abs() <= x.double().abs() * (2 ** -4 + 2 ** -19) + s.double() * 2 ** -10).all())
 
 
 @pytest.mark.parametrize("rows,h", [(1, 128), (3, 256), (77, 768), (33, 2880), (129, 7168), (5, 16384), (4, 16512)])
@@ -18,12 +19,12 @@ def test_row_and_block_scales(rows, h):
     x = torch.randn(rows, h, generator=g, device="cuda").bfloat16()
     x[0, :128] = 0
     q, s = cuda.quant_rowwise(x)
-    _same_up_to_a_step(q, s[:, None], x)
+    _rounded_to_nearest(q, s[:, None], x)
     assert torch.equal(s, x.abs().amax(-1).float().clamp_min(1e-12) / 448) or \
         bool((s * 448 / x.abs().amax(-1).float() - 1).abs().max() < 1e-6)
     if h % 128 == 0:
         q, s = cuda.quant_1x128(x)
-        _same_up_to_a_step(q, s.repeat_interleave(128, -1), x)
+        _rounded_to_nearest(q, s.repeat_interleave(128, -1), x)
         odd = torch.empty(rows * h + 4, device="cuda", dtype=torch.bfloat16)[4:].view(rows, h).copy_(x)   # 8-byte aligned
         qo, so = cuda.quant_1x128(odd)
         assert torch.equal(q.view(torch.uint8), qo.view(torch.uint8)) and torch.equal(s, so)

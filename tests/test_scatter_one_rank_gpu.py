@@ -38,9 +38,10 @@ def test_rows_scales_scalars_and_padding(tokens, topk, experts, hidden, fp8, sca
             q, s = cuda.quant_1x128(x)
             assert torch.equal(d.rows_fp8.view(torch.uint8)[rows], q.view(torch.uint8)[:, None, :].expand(tokens, topk, hidden))
             assert torch.equal(d.row_scales[rows], s[:, None, :].expand(tokens, topk, hidden // 128))
-        else:                                        # half an e4m3 step (2^-4), doubled for the kernel's reciprocal
-            got = d.rows_fp8[rows].float() * d.row_scales[rows].repeat_interleave(128, -1)
-            assert bool(((got - want).abs() <= want.abs() * 2 ** -3 + d.row_scales[rows].repeat_interleave(128, -1) * 2 ** -9).all())
+        else:                                        # half an e4m3 step, and 2^-19 for products and reciprocal in fp32
+            unit = d.row_scales[rows].repeat_interleave(128, -1)
+            got = d.rows_fp8[rows].float() * unit
+            assert bool(((got - want).abs() <= want.abs() * (2 ** -4 + 2 ** -19) + unit * 2 ** -10).all())
         assert torch.equal(d.scalars[0][rows], p)
         free = torch.ones(used, dtype=torch.bool, device="cuda")
         free[rows.reshape(-1)] = False
