@@ -63,11 +63,11 @@ def main(argv=None) -> int:
         y, dx, dw = torch.empty(r, n, device=dev, dtype=torch.bfloat16), torch.empty_like(x), torch.empty_like(w)
         flops = 2.0 * r * k * n
         ops = {
-            "fwd": (lambda: cops.grouped_gemm_raw(0, x, w, off, cnt, n, k, out=y, block_n=cops._pick_bn(n)),
+            "fwd": (lambda: cops.grouped_gemm_raw(0, x, w, off, cnt, n, k, out=y),
                     lambda: torch.matmul(x, w.t(), out=y)),
-            "dgrad": (lambda: cops.grouped_gemm_raw(1, g, w, off, cnt, n, k, out=dx, block_n=cops._pick_bn(k)),
+            "dgrad": (lambda: cops.grouped_gemm_raw(1, g, w, off, cnt, n, k, out=dx),
                       lambda: torch.matmul(g, w, out=dx)),
-            "wgrad": (lambda: cops.grouped_gemm_raw(2, g, x, off, cnt, n, k, out=dw, block_n=cops._pick_bn(k)),
+            "wgrad": (lambda: cops.grouped_gemm_raw(2, g, x, off, cnt, n, k, out=dw),
                       lambda: torch.matmul(g.t(), x, out=dw)),
         }
         for op, (own, lib) in ops.items():

@@ -132,13 +132,12 @@ class _GemmRS(torch.autograd.Function):
         da = dw = None
         if ctx.needs_input_grad[0]:
             da = torch.empty(ctx.a_shape, dtype=torch.bfloat16, device=g.device)
-            cops.grouped_gemm_raw(1, g_full, w, off, cnt, n, k, out=da.view(-1, k), block_n=cops._pick_bn(k))
+            cops.grouped_gemm_raw(1, g_full, w, off, cnt, n, k, out=da.view(-1, k))
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.w_ref, "main_grad", None)
             if mg is not None:             # straight into the flat gradient buffer of the parameter's group
-                cops.grouped_gemm_raw(2, g_full, a2, off, cnt, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written,
-                                      block_n=cops._pick_bn(k))
+                cops.grouped_gemm_raw(2, g_full, a2, off, cnt, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written)
                 ctx.w_ref.main_grad_written = True
             else:
-                dw = cops.grouped_gemm_raw(2, g_full, a2, off, cnt, n, k, block_n=cops._pick_bn(k)).view(n, k)
+                dw = cops.grouped_gemm_raw(2, g_full, a2, off, cnt, n, k).view(n, k)
         return da, dw, None

@@ -732,16 +732,14 @@ extern "C" unsigned long long slab_moe_wait_limit_ns();
 
 // mode: 0 fwd, 1 dgrad, 2 wgrad.  Shapes: see the header comment.  Requires K % 64 == 0, N % 64 == 0, at most 512
 // experts.  `status` is a device int the kernel sets on a bounded-wait timeout (0 = ok).  Returns a CUDA/driver error code
-// (0 = launched).  `max_ctas` > 0 bounds the CTAs (rounded down to pairs, at least one pair); `block_n`, a tile width the
-// caller would like, has no meaning here.
+// (0 = launched).  `max_ctas` > 0 bounds the CTAs (rounded down to pairs, at least one pair).
 // `ready` (optional, modes 0 and 1): per-(source, expert) arrival flags of the row operand, int [ready_world][E] in
 // this GPU's memory; the kernel waits (bounded) for all `ready_world` flags of an expert to reach `ready_epoch`
 // before it loads that expert's rows.  Null: the operand is complete when the kernel starts.
 extern "C" int slab_grouped_gemm_bf16(int mode, const void* A, const void* B, void* C, const int* seg_offsets,
-                                      const int* seg_counts, int E, int R, int N, int K, int accumulate, int block_n,
+                                      const int* seg_counts, int E, int R, int N, int K, int accumulate,
                                       int max_ctas, const int* ready, int ready_world, int ready_epoch, int* status,
                                       cudaStream_t stream) {
-  (void)block_n;
   using namespace slab;
   if (E > 512 || K % 64 || N % 64) return -100;
   if (ready && (ready_world < 1 || ready_world > 32 || mode == PG_WGRAD)) return -102;

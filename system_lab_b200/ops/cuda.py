@@ -37,7 +37,7 @@ _SIGS = {
     "slab_ce_fwd": "pppiis",
     "slab_scale_bf16": "plps",
     "slab_quant_tensorwise": "ppppls",
-    "slab_grouped_gemm_bf16": "i" + "p" * 5 + "i" * 7 + "pii" + "ps",
+    "slab_grouped_gemm_bf16": "i" + "p" * 5 + "i" * 6 + "pii" + "ps",
     "slab_grouped_gemm_fp8": "p" * 7 + "iiiii" + "ps",
     "slab_grouped_gemm_fp8_rowwise": "p" * 7 + "iiiii" + "ps",
 }
@@ -454,13 +454,12 @@ def _check_segments(offsets, counts):
 
 
 def grouped_gemm_raw(mode: int, a, b, offsets, counts, n: int, k: int, out=None, accumulate=False,
-                     block_n: int = 256, max_ctas: int = 0, ready=None):
+                     max_ctas: int = 0, ready=None):
     """mode 0: out[R,N] = a[R,K] @ b[e]^T ; 1: out[R,K] = a[R,N] @ b[e] ; 2: out[E,N,K] = a[R,N]^T @ b[R,K].
 
     ``ready`` (modes 0 and 1): arrival flags of the row operand (an object with ``flags`` int32 [world, E], ``world``,
     ``epoch`` and ``mark_consumed()``): the kernel waits per expert for every source instead of the caller waiting
-    for the whole exchange.  ``block_n`` is the tile width of the one-CTA kernel behind pushed results; the kernel here
-    picks its own tiles."""
+    for the whole exchange."""
     e = offsets.numel()
     r = a.shape[0]
     if out is None:
@@ -472,7 +471,7 @@ def grouped_gemm_raw(mode: int, a, b, offsets, counts, n: int, k: int, out=None,
             out = torch.empty(e, n, k, dtype=torch.bfloat16, device=a.device)
     if ready is not None and mode != 2:
         call("slab_grouped_gemm_bf16", mode, a, b, out, offsets, counts, e, r, n, k, 1 if accumulate else 0,
-             block_n, int(getattr(ready, "gemm_max_ctas", 0) or max_ctas), ready.flags, int(ready.world),
+             int(getattr(ready, "gemm_max_ctas", 0) or max_ctas), ready.flags, int(ready.world),
              int(ready.epoch), status_word(a.device), stream())
         ready.mark_consumed()
         ready.d.join_side()              # the remote half of the exchange, held back until this launch, starts now
@@ -480,7 +479,7 @@ def grouped_gemm_raw(mode: int, a, b, offsets, counts, n: int, k: int, out=None,
     if ready is not None:
         ready.wait()
     call("slab_grouped_gemm_bf16", mode, a, b, out, offsets, counts, e, r, n, k, 1 if accumulate else 0,
-         block_n, max_ctas, None, 0, 0, status_word(a.device), stream())
+         max_ctas, None, 0, 0, status_word(a.device), stream())
     return out
 
 
@@ -510,6 +509,7 @@ def grouped_gemm_fp8_rowwise_raw(a_q, sa, b_q, sb, offsets, counts, out=None, ma
 
 
 def _pick_bn(cols: int) -> int:
+    """Tile width of the one-CTA kernel (pushed results, gathered weights)."""
     return 256 if cols % 256 == 0 or cols > 1024 else 128
 
 
@@ -541,7 +541,7 @@ class _GroupedLinear(torch.autograd.Function):
                 push.launch(0, a, w, offsets, counts, n, k, _pick_bn(n))
             out = out if out is not None else torch.empty(1, dtype=torch.bfloat16, device=a.device).expand(a.shape[0], n)
         else:
-            out = grouped_gemm_raw(0, a, w, offsets, counts, n, k, out=out, block_n=_pick_bn(n), ready=ready)
+            out = grouped_gemm_raw(0, a, w, offsets, counts, n, k, out=out, ready=ready)
         ctx.save_for_backward(a, w, offsets, counts)
         ctx.w_ref = w
         ctx.dgrad_out = dgrad_out
@@ -573,7 +573,7 @@ class _GroupedLinear(torch.autograd.Function):
             else:
                 if do is not None and (do.shape[0] < g.shape[0] or do.shape[1] != k):
                     do = None
-                da = grouped_gemm_raw(1, g, w, offsets, counts, n, k, out=do, block_n=_pick_bn(k), ready=rdy)
+                da = grouped_gemm_raw(1, g, w, offsets, counts, n, k, out=do, ready=rdy)
                 rdy = None
                 if src is not None:
                     src.join_side()          # the side-stream half of the gradient scatter, if there was one
@@ -584,11 +584,10 @@ class _GroupedLinear(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.w_ref, "main_grad", None)
             if mg is not None:
-                grouped_gemm_raw(2, g, a, offsets, counts, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written,
-                                 block_n=_pick_bn(k))
+                grouped_gemm_raw(2, g, a, offsets, counts, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written)
                 ctx.w_ref.main_grad_written = True
             else:
-                dw = grouped_gemm_raw(2, g, a, offsets, counts, n, k, block_n=_pick_bn(k))
+                dw = grouped_gemm_raw(2, g, a, offsets, counts, n, k)
         return da, dw, None, None, None, None, None, None, None
 
 
@@ -676,11 +675,10 @@ class _GroupedLinearFp8(torch.autograd.Function):
             if ctx.needs_input_grad[1]:
                 mg = getattr(ctx.w_ref, "main_grad", None)
                 if mg is not None:
-                    grouped_gemm_raw(2, g, a, offsets, counts, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written,
-                                     block_n=_pick_bn(k))
+                    grouped_gemm_raw(2, g, a, offsets, counts, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written)
                     ctx.w_ref.main_grad_written = True
                 else:
-                    dw = grouped_gemm_raw(2, g, a, offsets, counts, n, k, block_n=_pick_bn(k))
+                    dw = grouped_gemm_raw(2, g, a, offsets, counts, n, k)
             return (da, dw) + (None,) * 7
         return _GroupedLinear.backward(ctx, g)          # same arity: (da, dw) + one None per remaining input
 
@@ -766,7 +764,7 @@ class _Linear(torch.autograd.Function):
             gather["comm"].gemm_gather(gather["ticket"], x2, w, out.view(-1, n), gather["flat"], gather["w_off"],
                                        (off, cnt), gather["pieces"], gather["call"], _pick_bn(n))
         else:
-            grouped_gemm_raw(0, x2, w, off, cnt, n, k, out=out.view(-1, n), block_n=_pick_bn(n))
+            grouped_gemm_raw(0, x2, w, off, cnt, n, k, out=out.view(-1, n))
         ctx.save_for_backward(x2, w, off, cnt)
         ctx.w_ref = w
         ctx.shp = shp
@@ -782,15 +780,14 @@ class _Linear(torch.autograd.Function):
         dx = dw = None
         if ctx.needs_input_grad[0]:
             dx = torch.empty(ctx.shp, dtype=torch.bfloat16, device=g.device)
-            grouped_gemm_raw(1, g2, w, off, cnt, n, k, out=dx.view(-1, k), block_n=_pick_bn(k))
+            grouped_gemm_raw(1, g2, w, off, cnt, n, k, out=dx.view(-1, k))
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.w_ref, "main_grad", None)
             if mg is not None:
-                grouped_gemm_raw(2, g2, x2, off, cnt, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written,
-                                 block_n=_pick_bn(k))
+                grouped_gemm_raw(2, g2, x2, off, cnt, n, k, out=mg, accumulate=ctx.w_ref.main_grad_written)
                 ctx.w_ref.main_grad_written = True
             else:
-                dw = grouped_gemm_raw(2, g2, x2, off, cnt, n, k, block_n=_pick_bn(k)).view(n, k)
+                dw = grouped_gemm_raw(2, g2, x2, off, cnt, n, k).view(n, k)
         return dx, dw, None
 
 
@@ -857,17 +854,17 @@ class _LinearCE(torch.autograd.Function):
             hi = min(lo + chunk_rows, n)
             off, cnt = _dense_segments(h.device, hi - lo)
             hc = h[lo:hi]
-            logits = grouped_gemm_raw(0, hc, weight, off, cnt, v, hd, block_n=256) if own else hc @ weight.t()
+            logits = grouped_gemm_raw(0, hc, weight, off, cnt, v, hd) if own else hc @ weight.t()
             if not (need_dh or need_dw):
                 call("slab_ce_fwd", logits, targets[lo:hi].contiguous(), loss_sum, hi - lo, v, stream())
                 continue
             call("slab_ce_fwd_bwd", logits, targets[lo:hi].contiguous(), loss_sum, hi - lo, v, gscale, stream())
             if need_dh and own:
-                grouped_gemm_raw(1, logits, weight, off, cnt, v, hd, out=dh[lo:hi], block_n=_pick_bn(hd))
+                grouped_gemm_raw(1, logits, weight, off, cnt, v, hd, out=dh[lo:hi])
             elif need_dh:
                 torch.mm(logits, weight, out=dh[lo:hi])
             if need_dw and own:
-                grouped_gemm_raw(2, logits, hc, off, cnt, v, hd, out=dw, accumulate=lo > 0, block_n=_pick_bn(hd))
+                grouped_gemm_raw(2, logits, hc, off, cnt, v, hd, out=dw, accumulate=lo > 0)
             elif need_dw:
                 dw.addmm_(logits.t(), hc)
         ctx.hooked = _saved_tensor_hooks_active()

@@ -39,46 +39,46 @@ CASES = [([128], 256, 128), ([100, 0, 300, 129], 512, 256), ([5, 700, 64, 1], 76
 
 
 @pytest.mark.parametrize("counts,n,k", CASES)
-@pytest.mark.parametrize("bn", [128, 256])
-def test_forward(counts, n, k, bn):
+@pytest.mark.parametrize("ctas", [0, 4])
+def test_forward(counts, n, k, ctas):
     from system_lab_b200.ops import cuda, reference as ref
     a, dy, w, off, cnt = _inputs(counts, n, k)
-    out = cuda.grouped_gemm_raw(0, a, w, off, cnt, n, k, block_n=bn)
+    out = cuda.grouped_gemm_raw(0, a, w, off, cnt, n, k, max_ctas=ctas)
     _check(out, ref.grouped_gemm(a, w, off, cnt), "fwd")
 
 
 @pytest.mark.parametrize("counts,n,k", CASES)
-@pytest.mark.parametrize("bn", [128, 256])
-def test_dgrad(counts, n, k, bn):
+@pytest.mark.parametrize("ctas", [0, 4])
+def test_dgrad(counts, n, k, ctas):
     from system_lab_b200.ops import cuda, reference as ref
     a, dy, w, off, cnt = _inputs(counts, n, k, 1)
-    out = cuda.grouped_gemm_raw(1, dy, w, off, cnt, n, k, block_n=bn)
+    out = cuda.grouped_gemm_raw(1, dy, w, off, cnt, n, k, max_ctas=ctas)
     _check(out, ref.grouped_gemm_dgrad(dy, w, off, cnt), "dgrad")
 
 
 @pytest.mark.parametrize("counts,n,k", CASES[:3])
-@pytest.mark.parametrize("bn", [128, 256])
-def test_wgrad(counts, n, k, bn):
+@pytest.mark.parametrize("ctas", [0, 4])
+def test_wgrad(counts, n, k, ctas):
     from system_lab_b200.ops import cuda, reference as ref
     a, dy, w, off, cnt = _inputs(counts, n, k, 2)
-    out = cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, block_n=bn)
+    out = cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, max_ctas=ctas)
     _check(out, ref.grouped_gemm_wgrad(dy, a, off, cnt), "wgrad")
     acc = out.clone()
-    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=acc, accumulate=True, block_n=bn)
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=acc, accumulate=True, max_ctas=ctas)
     _check(acc, 2 * ref.grouped_gemm_wgrad(dy, a, off, cnt).float(), "wgrad accumulate")
 
 
 @pytest.mark.parametrize("counts,n,k", [([130, 250], 2880, 192), ([64, 0, 300], 192, 320)])
-@pytest.mark.parametrize("bn", [128, 256])
-def test_wgrad_partial_row_tile(counts, n, k, bn):
+@pytest.mark.parametrize("ctas", [0, 4])
+def test_wgrad_partial_row_tile(counts, n, k, ctas):
     """N % 128 == 64 (hidden 2880): the last 64 rows of every expert's gradient come from a tile that hangs over
     the expert boundary; it must be written in full and must not touch the next expert's rows."""
     from system_lab_b200.ops import cuda, reference as ref
     a, dy, w, off, cnt = _inputs(counts, n, k, 2)
-    out = cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, block_n=bn)
+    out = cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, max_ctas=ctas)
     _check(out, ref.grouped_gemm_wgrad(dy, a, off, cnt), "wgrad partial")
     acc = out.clone()
-    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=acc, accumulate=True, block_n=bn)
+    cuda.grouped_gemm_raw(2, dy, a, off, cnt, n, k, out=acc, accumulate=True, max_ctas=ctas)
     _check(acc, 2 * ref.grouped_gemm_wgrad(dy, a, off, cnt).float(), "wgrad partial accumulate")
 
 

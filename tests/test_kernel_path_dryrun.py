@@ -34,7 +34,7 @@ def dry(monkeypatch):
             if isinstance(a, torch.Tensor) and a.dtype in (torch.int32, torch.int64):
                 a.data.zero_()
         calls.append(name)
-        if name == "slab_grouped_gemm_bf16" and args[13] is not None:
+        if name == "slab_grouped_gemm_bf16" and args[12] is not None:
             calls.waited_in_kernel += 1               # the GEMM took per-expert arrival flags
         cops.LAUNCHES[0] += 1
         return 0
