@@ -248,7 +248,7 @@ __device__ __forceinline__ void pg_uniform(PairTile& ti) {
 
 // Largest chunk (in 32-row units): the one whose waves of tiles cost least, the mean tile of n columns taken as n + 96: a
 // 64-deep step of n columns takes 249 ns at 128 and 398 ns at 256, because the weights' half of the operands is staged
-// whatever n is.  Over 78 products (13 dense and 11 grouped shapes, 128 to 20000 rows, forward and input gradient) the choice is
+// whatever n is.  Over 166 products (13 dense and 11 grouped shapes of 128 to 20000 rows, forward and input gradient) the choice is
 // within 0.3 % of the best of all eight in the mean and 5 % at worst; with n + 32 it was 2.1 % and 26 % (input gradient of
 // [4096, 7168] x [2048, 7168] 108.8 us in chunks of 160 where 256 take 90.3).
 // One warp; writes the segments and the tile prefix over experts, and returns the choice and a bound on the chunks it makes.
