@@ -450,8 +450,10 @@ template <bool GRAD>
 static int launch_ce(void* logits, const long* targets, float* loss_sum, int rows, int V, float gscale, cudaStream_t st) {
   if (V % 8) return -100;
   if (rows == 0) return 0;
-  // rows of up to 32 K columns leave most of 1024 threads without work: four smaller blocks share the SM
-  if (V > 32768)
+  // Two blocks per row pay where a row is long, or where there are not enough rows to give every SM two: 3095 rows of 33024 / 64000 /
+  // 96000 / 129280 columns 145 / 225 / 316 / 409 us, four small blocks per SM 95 / 206 / 319 / 426; 200 rows 13.2 / 18.3 / 24.7 /
+  // 34.3 against 12.2 / 19.9 / 28.3 / 41.8.
+  if (V > 98304 || (V > 49152 && rows <= 2 * 148))
     ce_kernel<512, 2, GRAD><<<2 * (rows < 148 ? rows : 148), 512, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
   else
     ce_kernel<256, 1, GRAD><<<rows < 148 * 4 ? rows : 148 * 4, 256, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
