@@ -855,10 +855,11 @@ static int launch_scatter(const void* x, const float* pair_scalar, const float* 
                           const int* expert_offsets, const int* expert_counts, int e_local, int pad, int fp8,
                           int* done_counter, int n_blocks, int eflags, cudaStream_t st) {
   if (H > 8192) return -100;                      // rows longer than 8192 columns are not covered
-  // Every block ends with a system fence and a count that all blocks share, so no more blocks than there are tokens for, one per
-  // warp, and between 3 and 8 per SM: 50 tokens and 32 experts (nearly all padding) 32 us with 8 per SM, 16 with 3 (e4m3), 8192
-  // tokens as with 8.  Measured on one rank; with peers as ever.
-  if (n_blocks <= 0) n_blocks = world == 1 ? min(max((T + 7) / 8, 148 * 3), 148 * 8) : 148 * 4;
+  // Every block ends with a system fence and a count that all blocks share.  3 blocks per SM do for what the L2 takes (rows and
+  // padding; 50 tokens and 32 experts, e4m3: 31 us with 8 per SM, 16 with 3; 500 tokens x 4096 and 64 experts 32 and 23), 8 are
+  // better for more (4096 tokens x 4096, top-4: 57 us with 3 to 4, 54 with 8).  Measured on one rank; with peers as ever.
+  const long bytes = ((long)T * K + (long)e_local * pad) * H * (fp8 ? 1 : 2);
+  if (n_blocks <= 0) n_blocks = 148 * (world > 1 ? 4 : bytes > (128L << 20) ? 8 : 3);
   auto kern = fp8 ? moe_scatter_kernel<true> : moe_scatter_kernel<false>;
   kern<<<n_blocks, 256, 0, st>>>((const __nv_bfloat16*)x, pair_scalar, scale_in, pair_loc, T, K, H, pt, ws, world, me, epoch,
                                  expert_offsets, expert_counts, e_local, pad, done_counter, eflags);
