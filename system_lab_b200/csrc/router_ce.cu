@@ -451,9 +451,9 @@ static int launch_ce(void* logits, const long* targets, float* loss_sum, int row
   if (V % 8) return -100;
   if (rows == 0) return 0;
   // Two blocks per row pay where a row is long, or where there are not enough rows to give every SM two: 3095 rows of 33024 / 64000 /
-  // 96000 / 129280 columns 145 / 225 / 316 / 409 us, four small blocks per SM 95 / 206 / 319 / 426; 200 rows 13.2 / 18.3 / 24.7 /
-  // 34.3 against 12.2 / 19.9 / 28.3 / 41.8.
-  if (V > 98304 || (V > 49152 && rows <= 2 * 148))
+  // 80000 / 96000 / 129280 columns 145 / 225 / 276 / 316 / 409 us, four small blocks per SM 95 / 206 / 262 / 319 / 426; 200 rows 13.2 /
+  // 18.3 / 21.9 / 24.7 / 34.3 against 12.2 / 19.9 / 24.1 / 28.3 / 41.8.
+  if (V > 90112 || (V > 49152 && rows <= 2 * 148))
     ce_kernel<512, 2, GRAD><<<2 * (rows < 148 ? rows : 148), 512, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
   else
     ce_kernel<256, 1, GRAD><<<rows < 148 * 4 ? rows : 148 * 4, 256, 0, st>>>((__nv_bfloat16*)logits, targets, loss_sum, rows, V, gscale);
